@@ -63,12 +63,22 @@ inline ClaimOrder claim_order(uint64_t n, uint64_t row, uint32_t shift = 3) {
 // the ray of `lane` in claim c, or n when the lane has none
 __device__ __forceinline__ uint64_t claimed_ray(const ClaimOrder& o, uint64_t c, uint32_t lane, uint64_t n) {
   if (c < o.blocks) {
-    const uint64_t band = c / o.per_band;
+    // a 64-bit division is a long sequence: claims that fit 32 bits take the short one
+    const uint64_t band = (o.blocks >> 32) ? c / o.per_band : (uint64_t)((uint32_t)c / (uint32_t)o.per_band);
     const uint64_t col = ((c - band * o.per_band) << o.shift) + (lane & ((1u << o.shift) - 1u));
     return col < o.row ? ((band << (5 - o.shift)) + (lane >> o.shift)) * o.row + col : n;
   }
   const uint64_t i = o.tail + (c - o.blocks) * 32 + lane;
   return i < n ? i : n;
+}
+
+// A warp has taken its last claim: the last of the launch's `warps` warps zeroes the claim counter
+// queue[0] and the count of finished warps queue[1] for the next launch on the stream.
+__device__ __forceinline__ void queue_done(unsigned long long* queue, uint64_t warps) {
+  if ((threadIdx.x & 31u) == 0u && atomicAdd(queue + 1, 1ull) == warps - 1u) {
+    queue[0] = 0;
+    queue[1] = 0;
+  }
 }
 
 // ------------------------------------------------------------------ Rust f32 semantics
@@ -177,9 +187,16 @@ __device__ __forceinline__ void impact_normal(const Bounds& c, float px, float p
   const float h = c.s * 0.5f;
   const float mx = (c.x + h) - px, my = (c.y + h) - py, mz = (c.z + h) - pz;
   const float m = rmax(rmax(fabsf(mx), fabsf(my)), fabsf(mz));
-  const float vx = fabsf(mx) == m ? -mx : 0.0f;
-  const float vy = fabsf(my) == m ? -my : 0.0f;
-  const float vz = fabsf(mz) == m ? -mz : 0.0f;
+  const bool ex = fabsf(mx) == m, ey = fabsf(my) == m, ez = fabsf(mz) == m;
+  // one largest component v gives v / sqrt(v * v) = +-1 exactly (v * v neither over- nor underflows in
+  // the range tested) and the others 0 / |v| = 0; ties (an edge) take the reference's operations
+  if (!((ex && ey) || (ex && ez) || (ey && ez)) && m > 0x1p-40f && m < 0x1p40f) {
+    nx = ex ? copysignf(1.0f, -mx) : 0.0f;
+    ny = ey ? copysignf(1.0f, -my) : 0.0f;
+    nz = ez ? copysignf(1.0f, -mz) : 0.0f;
+    return;
+  }
+  const float vx = ex ? -mx : 0.0f, vy = ey ? -my : 0.0f, vz = ez ? -mz : 0.0f;
   const float len = sqrtf((vx * vx + vy * vy) + vz * vz);
   nx = vx / len;
   ny = vy / len;
@@ -476,7 +493,7 @@ __device__ void cast_ray(const SceneView& s, const SharedLuts& L, float ox, floa
 // 2^-22 |p|) of p_j, so the condition is false while (L + j - 1)(vd - sqrt(3)) exceeds
 // |o - p| + j g + sqrt(3) 2^-21 S, padded by 2^-20 for the f32 evaluation.  Both sides grow
 // linearly in j, so the first visit and the slopes decide.  Evaluated in f64.
-static __device__ __noinline__ bool lod_runs_clear(float ox, float oy, float oz, float px, float py, float pz, float cx,
+static __host__ __device__ __noinline__ bool lod_runs_clear(float ox, float oy, float oz, float px, float py, float pz, float cx,
                                             float cy, float cz, float level, float viewing_distance, float S) {
   if (!(level > 0.0f) || !(viewing_distance > 0.0f)) return false;
   const double pad = 1.0 + 0x1p-20, r3 = 1.7320508075688772 * pad;
@@ -614,11 +631,10 @@ __device__ __forceinline__ uint32_t probe_brick_fast(const SceneView& s, FastRay
   }
 }
 
-// probe of a node's MIP brick (kind in meta[25:24]; kind 3: no node_mips entry, where the reference panics)
+// probe of a node's MIP brick (kind 3: no node_mips entry, where the reference panics)
 template <bool kCount>
-__device__ __forceinline__ uint32_t probe_mip(const SceneView& s, FastRay& r, uint32_t meta, uint32_t value,
+__device__ __forceinline__ uint32_t probe_mip(const SceneView& s, FastRay& r, uint32_t mk, uint32_t value,
                                               const Bounds& b, HitRecord& h, uint32_t& work) {
-  const uint32_t mk = (meta >> 24) & 3u;
   if (mk == 3u) return 3;
   return probe_brick_fast<kCount>(s, r, mk, value, b, h, work);
 }
@@ -626,7 +642,7 @@ __device__ __forceinline__ uint32_t probe_mip(const SceneView& s, FastRay& r, ui
 // kLod: get_by_ray_at_lod with MIP maps (s.mips): the MIP reads of the literal form, and restart
 // runs taken in closed form only where lod_runs_clear proves that none of their visits reads a MIP.
 // The record of a ray that hits nothing.
-__device__ __forceinline__ void miss_record(HitRecord& h) {
+__host__ __device__ __forceinline__ void miss_record(HitRecord& h) {
   h.status = 0;
   h.octant = 0;
   h.node = 0;
@@ -654,11 +670,13 @@ __device__ __forceinline__ bool fast_entry(const SceneView& s, float ox, float o
                 (oz < lo && dz < 0.0f) || (oz > S && dz > 0.0f)))
       return false;
   }
+  // fminf and fmaxf ignore a NaN like Rust's f32::min and max; they may pick the other zero of +-0, which
+  // moves the entry point by d * +-0: nothing but the sign of a coordinate that is 0
   const float t1 = (0.0f - ox) / dx, t2 = ((0.0f + S) - ox) / dx;
   const float t3 = (0.0f - oy) / dy, t4 = ((0.0f + S) - oy) / dy;
   const float t5 = (0.0f - oz) / dz, t6 = ((0.0f + S) - oz) / dz;
-  const float tmin = rmax(rmax(rmin(t1, t2), rmin(t3, t4)), rmin(t5, t6));
-  const float tmax = rmin(rmin(rmax(t1, t2), rmax(t3, t4)), rmax(t5, t6));
+  const float tmin = fmaxf(fmaxf(fminf(t1, t2), fminf(t3, t4)), fminf(t5, t6));
+  const float tmax = fminf(fminf(fmaxf(t1, t2), fmaxf(t3, t4)), fmaxf(t5, t6));
   if (tmax < 0.0f || tmin > tmax) return false;
   const float t = tmin < 0.0f ? 0.0f : tmin;
   px = ox + dx * t;
@@ -686,7 +704,10 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
   r.pos = (rsignum(dx) > 0.0f ? 1u : 0u) | (rsignum(dz) > 0.0f ? 2u : 0u) | (rsignum(dy) > 0.0f ? 4u : 0u);
   const float g4x = (r.pos & 1u) ? 4.0f : -4.0f, g4y = (r.pos & 4u) ? 4.0f : -4.0f, g4z = (r.pos & 2u) ? 4.0f : -4.0f;
   const uint32_t dir = hash_region(1.0f + dx, 1.0f + dy, 1.0f + dz, 1.0f);
-  const uint64_t* rtn = L.ray_to_node + dir;
+  const uint64_t* rtn = kStage ? L.ray_to_node + dir : nullptr;
+  // the nodes' heads as the direction octant sees them, and how they mirror octants and bitmap cells
+  const uint4* heads = s.heads + (size_t)dir * s.head_stride;
+  const uint32_t flip = dir ^ 7u, flip_cells = (flip & 1u) * 3u + (flip & 4u) * 3u + (flip & 2u) * 24u;
   const float S = s.size;
   Bounds cb{0.0f, 0.0f, 0.0f, S, s.inv_size};
   r.px = px;
@@ -717,14 +738,26 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
       const bool staged = kStage && (cur & kStagedBit) != 0u;
       const DevNode* nd = s.nodes + cur;
       const DevNode* sn = kStage ? stg + (cur & ~kStagedBit) : nd;
-      const uint4 head = staged ? *reinterpret_cast<const uint4*>(sn) : __ldg(reinterpret_cast<const uint4*>(nd));
+      // the head: occupancy and kinds from the record (kStage), or what they say to this direction
+      const uint4 head = kStage ? (staged ? *reinterpret_cast<const uint4*>(sn) : __ldg(reinterpret_cast<const uint4*>(nd)))
+                                : __ldg(heads + cur);
       const uint64_t occ = ((uint64_t)head.y << 32) | head.x;
       const uint32_t meta = head.z;
-      const uint32_t kind = meta & 3u;
+      const uint32_t kind = kStage ? meta & 3u : (meta >> 16) & 3u;
       const bool uniform = kind == kKindUniform;
-      const bool backtrack = uniform;  // a UniformLeaf is always left after its probe
+      // an octant that pushes or stops an ADVANCE (occupied with a child, a brick that is not Empty)
+      auto live = [&](uint32_t o) {
+        if (!kStage) return ((meta >> (o ^ flip)) & 1u) != 0u;
+        return kind == kKindInternal ? (occ & L.octant[o]) != 0 : kind == kKindLeaf && ((meta >> (8 + 2 * o)) & 3u) != kBkEmpty;
+      };
+      // anything between bitmap cell `flat` and the far corner; a UniformLeaf is always left after its probe
+      auto reaches = [&](uint32_t flat) {
+        if (kStage) return !uniform && (occ & rtn[flat * 8u]) != 0;
+        const uint32_t c = flat ^ flip_cells;
+        return ((((c & 32u) ? head.y : head.x) >> (c & 31u)) & 1u) != 0u;
+      };
       if (lod && lod_reads_mip(ox, oy, oz, r.px, r.py, r.pz, mip_level, viewing_distance)) {
-        const uint32_t rc = probe_mip<kCount>(s, r, meta, head.w, cb, h, work);
+        const uint32_t rc = probe_mip<kCount>(s, r, (meta >> 18) & 3u, head.w, cb, h, work);
         if (rc) {
           h.status = rc;
           h.node = cur;
@@ -735,7 +768,8 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
       if (target != kOob && (uniform || kind == kKindLeaf)) {
         // probe the UniformLeaf's brick over the node bounds, or the Leaf's brick under target_octant
         const uint32_t slot = uniform ? 0u : target;
-        const uint32_t bk = (meta >> (8 + 2 * slot)) & 3u;
+        const uint32_t bk = kStage ? (meta >> (8 + 2 * slot)) & 3u
+                            : !live(target) ? kBkEmpty : ((meta >> (8u + (target ^ flip))) & 1u) ? kBkSolid : kBkParted;
         if (bk != kBkEmpty) {
           const uint32_t rc = probe_brick_fast<kCount>(s, r, bk, __ldg(&nd->slot[slot]),
                                                        uniform ? cb : child_bounds(cb, target), h, work);
@@ -754,7 +788,7 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
       const float rz = (r.pz - cb.z) * q4;
       uint32_t flat = min(__float2uint_rz(rx), 3u) + 4u * min(__float2uint_rz(ry), 3u) +
                       16u * min(__float2uint_rz(rz), 3u);
-      if (backtrack || target == kOob || occ == 0 || (occ & rtn[flat * 8u]) == 0) {
+      if (target == kOob || !reaches(flat)) {
         // POP.  The popped node was pushed as child `ho` of the new top, so its bounds are
         // child_bounds_for(parent, ho): the reference's parent minimum min - fmod(min, 2 size) is
         // min - offset(ho) * size and hash_region(center - parent_min, size) is ho (both exact).
@@ -781,7 +815,7 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
       // the child key is read only where the octant is occupied: an empty octant neither pushes nor
       // stops an ADVANCE, whatever its key
       uint32_t ck = kInvalidChild;
-      if (kind == kKindInternal && (occ & L.octant[target]) != 0) ck = staged ? sn->slot[target] : __ldg(&nd->slot[target]);
+      if (kind == kKindInternal && live(target)) ck = staged ? sn->slot[target] : __ldg(&nd->slot[target]);
       if (ck != kInvalidChild) {
         // PUSH (the child's octant in its parent rides along: 3 bits per stack entry); a staged
         // node's staged child is entered through its copy
@@ -825,11 +859,13 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
             return;
           }
           flat = ux + 4u * uy + 16u * uz;
-          if (kind == kKindInternal && (occ & L.octant[target]) != 0 && (rtn[flat * 8u] & occ) != 0) {
-            ck = staged ? sn->slot[target] : __ldg(&nd->slot[target]);
-            if (ck != kInvalidChild) break;
+          if (live(target)) {
+            if (kind == kKindLeaf) break;
+            if (reaches(flat)) {
+              ck = staged ? sn->slot[target] : __ldg(&nd->slot[target]);
+              if (ck != kInvalidChild) break;
+            }
           }
-          if (kind == kKindLeaf && ((meta >> (8 + 2 * target)) & 3u) != kBkEmpty) break;
         }
       }
     }
@@ -840,9 +876,10 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
     // Restarts whose root visit fails its occupancy test (an Internal or empty root, whose visit
     // neither probes nor pushes) repeat visit, POP and nudge until the point changes root bitmap
     // cell; each such run is taken in closed form, counting its visits.
-    const uint4 root = __ldg(reinterpret_cast<const uint4*>(s.nodes));
+    const uint4 root = kStage ? __ldg(reinterpret_cast<const uint4*>(s.nodes)) : __ldg(heads);
     const uint64_t occ_root = ((uint64_t)root.y << 32) | root.x;
-    const bool root_runs = (root.z & 3u) == kKindInternal || (root.z & 3u) == kKindNothing;
+    const uint32_t root_kind = kStage ? root.z & 3u : (root.z >> 16) & 3u;
+    const bool root_runs = root_kind == kKindInternal || root_kind == kKindNothing;
     const float q4r = s.inv_size * 4.0f;
     while (root_runs && r.px < S && r.py < S && r.pz < S && r.px > 0.0f && r.py > 0.0f && r.pz > 0.0f) {
       // a root visit that reads the root's MIP (which may move the point before the occupancy
@@ -851,7 +888,9 @@ __device__ void cast_ray_fast_from(const SceneView& s, const SharedLuts& L, floa
       const float rx = (r.px - 0.0f) * q4r, ry = (r.py - 0.0f) * q4r, rz = (r.pz - 0.0f) * q4r;
       const uint32_t flat = min(__float2uint_rz(rx), 3u) + 4u * min(__float2uint_rz(ry), 3u) +
                             16u * min(__float2uint_rz(rz), 3u);
-      if (occ_root != 0 && (occ_root & rtn[flat * 8u]) != 0) break;
+      if (kStage ? (occ_root & rtn[flat * 8u]) != 0
+                 : (((((flat ^ flip_cells) & 32u) ? root.y : root.x) >> ((flat ^ flip_cells) & 31u)) & 1u) != 0u)
+        break;
       if (++work > kWorkCap) {
         h.status = 2;
         return;

@@ -17,6 +17,7 @@
 #include "svo_queue.h"
 #include "svo_refill.cuh"
 #include "svo_trace.h"
+#include "svo_unit.cuh"
 
 namespace svo {
 
@@ -69,15 +70,15 @@ void image_free(void* p) {
     cudaFree(p);
 }
 
+// One ray per lane, 1 << lanes rays per warp.
 template <bool kCount>
-__global__ void __launch_bounds__(128, 7) cast_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n) {
-  __shared__ SharedLuts L;
-  fill_shared_luts(L);
-  __syncthreads();
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__global__ void __launch_bounds__(128, 7)
+    cast_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, uint32_t lanes) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t i = (((uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5)) << lanes) + lane;
+  if (lane >> lanes || i >= n) return;
   HitRecord h;
-  cast_one<kCount>(s, L, __ldg(rays.ox + i), __ldg(rays.oy + i), __ldg(rays.oz + i), __ldg(rays.dx + i),
+  cast_one<kCount>(s, kLuts, __ldg(rays.ox + i), __ldg(rays.oy + i), __ldg(rays.oz + i), __ldg(rays.dx + i),
                    __ldg(rays.dy + i), __ldg(rays.dz + i), h);
   write_hit(s, out, i, h);
   if (kCount) write_counters(out, i, h);
@@ -86,7 +87,8 @@ __global__ void __launch_bounds__(128, 7) cast_kernel(SceneView s, RaysView rays
 // Queued cast: a persistent grid whose warps claim 32 rays at a time from a work counter.  The
 // cost of a ray varies by orders of magnitude (a sky ray leaves after a few node visits, a
 // grazing ray walks a whole cave), and a warp that finishes early takes more work instead of
-// idling until its block's slowest warp is done.  The counter (claims taken) starts at 0.
+// idling until its block's slowest warp is done.  The counter (claims taken) starts at 0, and the last
+// warp to finish zeroes it for the next launch (queue_done).
 //
 // Rays that miss the octree's root box get their miss written at once.  A claim whose rays all
 // enter is cast as it is; the entering rays of other claims wait in the warp's slice of shared
@@ -101,16 +103,10 @@ struct WaitingRays {  // the ray's origin and direction are read again from the 
 // kStage: the block first copies the scene's top table's first stage_n records into dynamic shared
 // memory, and the fast form reads those nodes there.
 template <bool kCount, bool kLod = false, bool kStage = false>
-__global__ void __launch_bounds__(128, 7)
-    queue_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                 unsigned long long* __restrict__ counter, float viewing_distance = 0.0f, uint32_t stage_n = 0) {
-  __shared__ SharedLuts L;
-  __shared__ WaitingRays waiting[4];
-  extern __shared__ uint4 staged_smem[];
-  DevNode* stg = reinterpret_cast<DevNode*>(staged_smem);
-  fill_shared_luts(L);
-  if (kStage) stage_records(stg, s.top, stage_n);
-  __syncthreads();
+__device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& rays, const HitsView& out, uint64_t n,
+                                           const ClaimOrder& order, unsigned long long* __restrict__ queue,
+                                           const SharedLuts& L, WaitingRays (&waiting)[4], const DevNode* stg,
+                                           float viewing_distance = 0.0f, uint32_t stage_n = 0) {
   const uint32_t lane = threadIdx.x & 31u;
   WaitingRays& w = waiting[threadIdx.x >> 5];
   uint32_t count = 0;  // rays waiting (the same in every lane)
@@ -122,7 +118,7 @@ __global__ void __launch_bounds__(128, 7)
     uint32_t target = 0;
     while (more && count < 32) {
       unsigned long long c = 0;
-      if (lane == 0) c = atomicAdd(counter, 1ull);
+      if (lane == 0) c = atomicAdd(queue, 1ull);
       c = __shfl_sync(0xFFFFFFFFu, c, 0);
       if (c >= order.claims) {
         more = false;
@@ -192,6 +188,25 @@ __global__ void __launch_bounds__(128, 7)
     write_hit(s, out, i, h);
     if (kCount) write_counters(out, i, h);
   }
+  queue_done(queue, (uint64_t)gridDim.x * 4u);
+}
+
+template <bool kCount, bool kLod = false, bool kStage = false>
+__global__ void __launch_bounds__(128, 7)
+    queue_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
+                 unsigned long long* __restrict__ queue, float viewing_distance = 0.0f, uint32_t stage_n = 0) {
+  __shared__ WaitingRays waiting[4];
+  if constexpr (kStage) {
+    __shared__ SharedLuts L;
+    extern __shared__ uint4 staged_smem[];
+    DevNode* stg = reinterpret_cast<DevNode*>(staged_smem);
+    fill_shared_luts(L);
+    stage_records(stg, s.top, stage_n);
+    __syncthreads();
+    queue_cast<kCount, kLod, kStage>(s, rays, out, n, order, queue, L, waiting, stg, viewing_distance, stage_n);
+  } else {
+    queue_cast<kCount, kLod>(s, rays, out, n, order, queue, kLuts, waiting, nullptr, viewing_distance);
+  }
 }
 
 // Refilling cast: the work queue of queue_kernel, where a warp also parks its rays at a node visit
@@ -202,7 +217,7 @@ __global__ void __launch_bounds__(128, 7)
 template <bool kCount, bool kStage = false>
 __global__ void __launch_bounds__(128, 7)
     refill_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                  unsigned long long* __restrict__ counter, uint32_t park_below, uint32_t stage_n = 0) {
+                  unsigned long long* __restrict__ queue, uint32_t park_below, uint32_t stage_n = 0) {
   __shared__ SharedLuts L;
   __shared__ WaitingRays waiting[4];
   __shared__ uint32_t in_flight[4];  // rays of each warp in flight (parked ones included)
@@ -229,7 +244,7 @@ __global__ void __launch_bounds__(128, 7)
       // claims until `need` entering rays wait or no claims are left (misses written at once)
       while (more && count < need) {
         unsigned long long c = 0;
-        if (lane == 0) c = atomicAdd(counter, 1ull);
+        if (lane == 0) c = atomicAdd(queue, 1ull);
         c = __shfl_sync(0xFFFFFFFFu, c, 0);
         if (c >= order.claims) {
           more = false;
@@ -306,6 +321,7 @@ __global__ void __launch_bounds__(128, 7)
     }
     __syncwarp();
   }
+  queue_done(queue, (uint64_t)gridDim.x * 4u);
 }
 
 // Host-buffer cast that reads its rays from and writes its hits to host memory in place (over the CPU
@@ -321,19 +337,13 @@ struct PairStage {  // one warp's two blocks, a field at a time (no bank conflic
 };
 
 __global__ void __launch_bounds__(128, 7)
-    pair_rows_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                     unsigned long long* __restrict__ counter) {
-  __shared__ SharedLuts L;
+    pair_rows_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
+                     unsigned long long* __restrict__ queue) {
   __shared__ PairStage stage[4];
-  fill_shared_luts(L);
-  __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
   PairStage& ps = stage[threadIdx.x >> 5];
-  for (;;) {
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(counter, 2ull);
-    c = __shfl_sync(0xFFFFFFFFu, c, 0);
-    if (c >= order.claims) break;
+  const uint64_t warps = (uint64_t)gridDim.x * 4u;
+  for (unsigned long long c = ((uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5)) * 2u; c < order.claims;) {
     for (uint32_t half = 0; half < 2; ++half) {
       const uint64_t cc = c + half;
       const uint64_t j = cc < order.claims ? claimed_ray(order, cc, lane, n) : n;
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(128, 7)
         float px = 0.0f, py = 0.0f, pz = 0.0f;
         uint32_t target = 0;
         if (!fast || fast_entry(s, ox, oy, oz, dx, dy, dz, px, py, pz, target))
-          cast_entered<false>(s, L, ox, oy, oz, dx, dy, dz, fast, px, py, pz, target, h);
+          cast_entered<false>(s, kLuts, ox, oy, oz, dx, dy, dz, fast, px, py, pz, target, h);
       }
       // write_hit's record, kept for the rows below
       uint32_t kind, albedo, user;
@@ -397,10 +407,17 @@ __global__ void __launch_bounds__(128, 7)
       }
     }
     __syncwarp();
+    if (lane == 0) c = atomicAdd(queue, 2ull) + 2u * warps;
+    c = __shfl_sync(0xFFFFFFFFu, c, 0);
   }
+  queue_done(queue, warps);
 }
 
-constexpr uint64_t kQueueMinRays = 1u << 15;  // below this the one-thread-per-ray grid is as fast
+// Below this many rays one grid with fewer rays per warp (grid_lanes) is faster than the work queue: 119,860 camera
+// rays on 512^3 135 us against 157, on 256^3 117 against 120; at 160,000 the two are even.
+constexpr uint64_t kQueueMinRays = 1u << 17;
+// The same line where the rays are read from host memory: the queue's 16 x 2 blocks read it in longer pieces.
+constexpr uint64_t kInPlaceMinRays = 1u << 15;
 
 void destroy_queues(DeviceImage& d) {
   if (!d.queues) return;
@@ -409,7 +426,7 @@ void destroy_queues(DeviceImage& d) {
   d.queues = nullptr;
 }
 
-svo_status create_queues(DeviceImage& d) {
+svo_status create_queues(DeviceImage& d, cudaStream_t st) {
   if (d.queues) return SVO_OK;
   CastQueues* q = new CastQueues();
   int dev = 0;
@@ -418,7 +435,8 @@ svo_status create_queues(DeviceImage& d) {
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm, queue_kernel<false>, 128, 0);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_count, queue_kernel<true>, 128, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&q->counters, kQueueSlots * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&q->counters, 2 * kQueueSlots * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMemsetAsync(q->counters, 0, 2 * kQueueSlots * sizeof(unsigned long long), st);
   if (e != cudaSuccess) {
     cudaFree(q->counters);
     delete q;
@@ -431,15 +449,12 @@ svo_status create_queues(DeviceImage& d) {
 
 // get_by_ray_at_lod one thread per ray, for streams without a work counter.
 template <bool kCount>
-__global__ void __launch_bounds__(128) lod_grid_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n,
+__global__ void __launch_bounds__(128) lod_grid_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n,
                                                        float viewing_distance) {
-  __shared__ SharedLuts L;
-  fill_shared_luts(L);
-  __syncthreads();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   HitRecord h;
-  cast_one<kCount, true>(s, L, __ldg(rays.ox + i), __ldg(rays.oy + i), __ldg(rays.oz + i), __ldg(rays.dx + i),
+  cast_one<kCount, true>(s, kLuts, __ldg(rays.ox + i), __ldg(rays.oy + i), __ldg(rays.oz + i), __ldg(rays.dx + i),
                          __ldg(rays.dy + i), __ldg(rays.dz + i), h, viewing_distance);
   write_hit(s, out, i, h);
   if (kCount) write_counters(out, i, h);
@@ -452,11 +467,22 @@ int g_refill_below = 0;   // svo_set_refill: a warp parks and refills below this
 int g_pair_rows = 1;      // host buffers read and written in place: 32 x 2 blocks written row by row
 
 // ------------------------------------------------------------------ device image
+// a node's record and its heads, one per direction octant
+constexpr uint64_t kNodeBytes = sizeof(DevNode) + kHeadPlanes * sizeof(uint4);
+
+// The heads of all node records, one thread per node and plane.  Bound by its traffic (64 bytes in, 128
+// out per node); the records are read once from DRAM, the other planes' reads hit L2.
+__global__ void __launch_bounds__(256) build_heads(const DevNode* __restrict__ nodes, uint32_t n,
+                                                   uint4* __restrict__ heads, uint32_t stride) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) heads[(size_t)blockIdx.y * stride + k] = node_head(nodes[k], blockIdx.y);
+}
+
 uint64_t device_image_bytes(const svo_scene* sc) {
   const DeviceImage& d = sc->dev;
   if (!d.valid) return 0;
   const uint64_t len = sc->tree.arena.len(), W = len >= 32 ? len / 32 : 1;
-  return d.node_cap * sizeof(DevNode) + d.brick_cap * (len + W) * 4 + (d.color_cap + d.data_cap) * 4 +
+  return d.node_cap * kNodeBytes + d.brick_cap * (len + W) * 4 + (d.color_cap + d.data_cap) * 4 +
          kMaxStaged * sizeof(DevNode);
 }
 uint64_t device_image_bytes_estimate(const svo_scene* sc) {
@@ -464,7 +490,7 @@ uint64_t device_image_bytes_estimate(const svo_scene* sc) {
   const uint64_t nn = t.nodes(), nb = std::max<uint64_t>(1, t.arena.slots());
   const uint64_t nc = std::max<uint64_t>(1, t.colors.size()), nd = std::max<uint64_t>(1, t.datas.size());
   const uint64_t len = t.arena.len(), W = len >= 32 ? len / 32 : 1;
-  return (nn + nn / 4 + 64) * sizeof(DevNode) + (nb + nb / 4 + 16) * (len + W) * 4 + (nc + nc / 4 + 64 + nd + nd / 4 + 64) * 4 +
+  return (nn + nn / 4 + 64) * kNodeBytes + (nb + nb / 4 + 16) * (len + W) * 4 + (nc + nc / 4 + 64 + nd + nd / 4 + 64) * 4 +
          kMaxStaged * sizeof(DevNode);
 }
 
@@ -491,6 +517,8 @@ SceneView scene_view(const svo_scene* sc) {
   for (uint32_t r = sc->tree.size / sc->tree.dim; r > 1; r >>= 1) ++levels;
   v.mip_top = (float)levels;
   v.top = d.top;
+  v.heads = d.heads;
+  v.head_stride = (uint32_t)d.node_cap;
   return v;
 }
 
@@ -500,6 +528,15 @@ uint32_t staged_records(const svo_scene* sc, uint32_t depth) {
 }
 
 namespace {
+
+// Writes the heads of the image's first `nn` nodes on st, after their records' copies.
+svo_status write_heads(DeviceImage& d, uint64_t nn, cudaStream_t st) {
+  if (nn == 0) return SVO_OK;
+  build_heads<<<dim3((unsigned)((nn + 255) / 256), kHeadPlanes), 256, 0, st>>>(d.nodes, (uint32_t)nn, d.heads,
+                                                                               (uint32_t)d.node_cap);
+  SVO_CUDA_TRY(cudaGetLastError());
+  return SVO_OK;
+}
 
 uint32_t vwords_of(const HostOctree& t) { return t.arena.len() >= 32 ? t.arena.len() / 32 : 1; }
 
@@ -645,6 +682,7 @@ void free_device(DeviceImage& d) {
   d.top = nullptr;
   for (auto& c : d.top_count) c = 0;  // top_keys describe the host mirror, which stays
   d.nodes = nullptr;
+  d.heads = nullptr;
   d.voxels = d.vbits = d.colors = d.datas = nullptr;
   d.node_cap = d.brick_cap = d.color_cap = d.data_cap = 0;
   d.valid = false;
@@ -719,7 +757,7 @@ svo_status upload_block(svo_scene* sc, cudaStream_t st, bool fill) {
   }
   void* p = nullptr;
   {
-    const svo_status rc = image_alloc(&p, total, st, true);
+    const svo_status rc = image_alloc(&p, total + d.node_cap * kHeadPlanes * sizeof(uint4), st, true);
     if (rc != SVO_OK) {
       d.ordered = false;
       free_device(d);
@@ -734,12 +772,17 @@ svo_status upload_block(svo_scene* sc, cudaStream_t st, bool fill) {
   d.vbits = reinterpret_cast<uint32_t*>(base + off[3]);
   d.colors = reinterpret_cast<uint32_t*>(base + off[4]);
   d.datas = reinterpret_cast<uint32_t*>(base + off[5]);
+  d.heads = reinterpret_cast<uint4*>(base + total);  // written on the device, no part of the blob
   const uint64_t used[6] = {t.nodes() * sizeof(DevNode), d.host_top.size() * sizeof(DevNode), nb * len * 4,
                             nb * W * 4, t.colors.size() * 4, t.datas.size() * 4};
   for (int i = 0; i < 6; ++i)
     if (used[i]) SVO_CUDA_TRY(cudaMemcpyAsync(base + off[i], d.blob + off[i], used[i], cudaMemcpyHostToDevice, st));
   if (!d.blob_done) SVO_CUDA_TRY(cudaEventCreateWithFlags(&d.blob_done, cudaEventDisableTiming));
   SVO_CUDA_TRY(cudaEventRecord(d.blob_done, st));
+  {
+    const svo_status rc = write_heads(d, t.nodes(), st);
+    if (rc != SVO_OK) return rc;
+  }
   image_synced(t, d);
   return SVO_OK;
 }
@@ -750,7 +793,7 @@ svo_status full_upload(svo_scene* sc, cudaStream_t st, bool ordered = false) {
   free_device(d);
   d.ordered = ordered && !caller_allocator();
   {
-    const svo_status qs = create_queues(d);
+    const svo_status qs = create_queues(d, st);
     if (qs != SVO_OK) return qs;
   }
   const uint64_t nn = t.nodes(), nb = std::max<uint64_t>(1, t.arena.slots());
@@ -791,7 +834,7 @@ svo_status full_upload(svo_scene* sc, cudaStream_t st, bool ordered = false) {
   {
     // a failed allocation releases what the upload holds: the scene is left without a device image
     void* p[5] = {};
-    const size_t bytes[5] = {d.node_cap * sizeof(DevNode), d.brick_cap * (size_t)len * 4, d.brick_cap * (size_t)W * 4,
+    const size_t bytes[5] = {d.node_cap * kNodeBytes, d.brick_cap * (size_t)len * 4, d.brick_cap * (size_t)W * 4,
                              d.color_cap * 4, d.data_cap * 4};
     for (int i = 0; i < 5; ++i) {
       const svo_status rc = image_alloc(&p[i], bytes[i], st, d.ordered);
@@ -808,12 +851,17 @@ svo_status full_upload(svo_scene* sc, cudaStream_t st, bool ordered = false) {
       }
     }
     d.nodes = static_cast<DevNode*>(p[0]);
+    d.heads = reinterpret_cast<uint4*>(d.nodes + d.node_cap);
     d.voxels = static_cast<uint32_t*>(p[1]);
     d.vbits = static_cast<uint32_t*>(p[2]);
     d.colors = static_cast<uint32_t*>(p[3]);
     d.datas = static_cast<uint32_t*>(p[4]);
   }
   SVO_CUDA_TRY(cudaMemcpyAsync(d.nodes, d.host_nodes.data(), nn * sizeof(DevNode), cudaMemcpyHostToDevice, st));
+  {
+    const svo_status hs = write_heads(d, nn, st);
+    if (hs != SVO_OK) return hs;
+  }
   {
     const svo_status ts = upload_top(d, st);
     if (ts != SVO_OK) {
@@ -874,12 +922,17 @@ svo_status incremental_sync(svo_scene* sc, cudaStream_t st) {
   } catch (const ReferencePanic& p) {
     return fail(SVO_ERR_REFERENCE_PANIC, std::string("sync: ") + p.what());
   }
+  const bool nodes_changed = std::find(t.node_dirty.begin(), t.node_dirty.end(), 1) != t.node_dirty.end();
   svo_status rc = copy_runs(t.node_dirty, nn, [&](uint64_t a, uint64_t b) -> svo_status {
     SVO_CUDA_TRY(cudaMemcpyAsync(d.nodes + a, d.host_nodes.data() + a, (b - a) * sizeof(DevNode),
                                  cudaMemcpyHostToDevice, st));
     return SVO_OK;
   });
   if (rc != SVO_OK) return rc;
+  if (nodes_changed) {
+    rc = write_heads(d, nn, st);
+    if (rc != SVO_OK) return rc;
+  }
   rc = upload_top(d, st);
   if (rc != SVO_OK) return rc;
   rc = copy_runs(t.arena.dirty(), t.arena.slots(), [&](uint64_t a, uint64_t b) -> svo_status {
@@ -906,6 +959,17 @@ svo_status incremental_sync(svo_scene* sc, cudaStream_t st) {
 }
 
 
+// Rays per warp (log2) of a batch that one grid casts, one ray per lane: 32 from 131,072 rays on, fewer for fewer
+// rays, so that there are 4,096 warps or more (about what is resident).  A warp takes the sum of its rays' different
+// steps, so more warps of fewer rays end sooner while they all run at once: 4,000 camera rays on 128^3 take
+// 41 us instead of 97, 1,000 random ones 26 instead of 45, 60,000 on 512^3 106 instead of 147 in the work queue.
+constexpr uint64_t kGridWarps = 4096;
+uint32_t grid_lanes(uint64_t n) {
+  uint32_t lanes = 5;
+  while (lanes > 0 && (n >> lanes) < kGridWarps) --lanes;
+  return lanes;
+}
+
 // `in_place`: rays and hits are host memory the device reads and writes through the CPU's page
 // tables; the claims are then 16 x 2 blocks (two 64-byte pieces of each array per warp instead of
 // four 32-byte ones), which the host link serves faster than 8 x 4 blocks.
@@ -918,19 +982,19 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
   const bool count = counts_requested(*hits);
   const unsigned block = 128;
   CastQueues* q = sc->dev.queues;
-  if (q && n >= kQueueMinRays) {
+  if (q && n >= (in_place ? kInPlaceMinRays : kQueueMinRays)) {
     std::lock_guard<std::mutex> lock(q->m);
-    if (unsigned long long* ctr = queue_counter(q, st)) {
+    if (unsigned long long* queue = queue_counter(q, st)) {
       const int per_sm = std::max(1, count ? q->blocks_per_sm_count : q->blocks_per_sm);
-      const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * per_sm, (n + block - 1) / block);
-      SVO_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st));
+      const uint64_t resident = (uint64_t)q->sm_count * per_sm;
       const ClaimOrder order = claim_order(n, row, in_place ? 4 : 3);
+      const uint64_t grid = std::min<uint64_t>(resident, (order.claims + 3) / 4);
       const uint32_t stage_n = g_cast_mode == 1 ? 0u : staged_records(sc, (uint32_t)g_stage_depth);
       // two blocks per claim halve the units of work: only where every resident warp gets at least four
       // of them (a small batch keeps the per-block claims, whose tail is shorter)
-      const uint64_t warps = (uint64_t)q->sm_count * (uint64_t)per_sm * (block / 32);
+      const uint64_t warps = resident * (block / 32);
       if (in_place && !count && stage_n == 0 && g_refill_below == 0 && g_pair_rows && n >= warps * 64 * 4) {
-        pair_rows_kernel<<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, ctr);
+        pair_rows_kernel<<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
       } else if (g_refill_below > 0) {
         const size_t smem = (size_t)stage_n * sizeof(DevNode);
         auto kern = stage_n ? (count ? refill_kernel<true, true> : refill_kernel<false, true>)
@@ -938,8 +1002,8 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         SVO_CUDA_TRY(allow_dynamic_smem(kern, smem));
         int per = 0;
         SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));
-        const uint64_t rgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (n + block - 1) / block);
-        kern<<<(unsigned)rgrid, block, smem, st>>>(v, rv, hv, n, order, ctr, (uint32_t)g_refill_below, stage_n);
+        const uint64_t rgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (order.claims + 3) / 4);
+        kern<<<(unsigned)rgrid, block, smem, st>>>(v, rv, hv, n, order, queue, (uint32_t)g_refill_below, stage_n);
       } else if (stage_n) {
         // the staged records take dynamic shared memory: resident blocks from this launch's size
         const size_t smem = (size_t)stage_n * sizeof(DevNode);
@@ -947,23 +1011,24 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         SVO_CUDA_TRY(allow_dynamic_smem(kern, smem));
         int per = 0;
         SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));
-        const uint64_t sgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (n + block - 1) / block);
-        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, ctr, 0.0f, stage_n);
+        const uint64_t sgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (order.claims + 3) / 4);
+        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n);
       } else if (count) {
-        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, ctr);
+        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
       } else {
-        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, ctr);
+        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
       }
       SVO_CUDA_TRY(cudaGetLastError());
       return SVO_OK;
     }
   }
-  const uint64_t grid = (n + block - 1) / block;
+  const uint32_t lanes = in_place ? 5u : grid_lanes(n);
+  const uint64_t grid = (((n + (1u << lanes) - 1) >> lanes) + 3) / 4;
   if (grid > 0x7FFFFFFFull) return fail(SVO_ERR_ARGUMENT, "svo_cast: too many rays for one launch");
   if (count)
-    cast_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n);
+    cast_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, lanes);
   else
-    cast_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n);
+    cast_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, lanes);
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }
@@ -1120,6 +1185,7 @@ svo_status evict_ordered(svo_scene* sc, cudaStream_t st) {
       if (p) SVO_CUDA_TRY(cudaFreeAsync(p, st));
   }
   d.top = d.nodes = nullptr;
+  d.heads = nullptr;
   d.voxels = d.vbits = d.colors = d.datas = nullptr;
   for (auto& c : d.top_count) c = 0;  // top_keys describe the host mirror, which stays
   d.node_cap = d.brick_cap = d.color_cap = d.data_cap = 0;
@@ -1206,8 +1272,8 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
   const HitsView hv = hits_view_of(*hits);
   const bool count = counts_requested(*hits);
   std::lock_guard<std::mutex> lock(q->m);
-  unsigned long long* ctr = queue_counter(q, st);
-  if (!ctr) {
+  unsigned long long* queue = queue_counter(q, st);
+  if (!queue) {
     const uint64_t blocks = (n + 127) / 128;
     if (blocks > 0x7FFFFFFFull) return fail(SVO_ERR_ARGUMENT, "svo_cast_lod: too many rays for one launch");
     if (count)
@@ -1221,13 +1287,12 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
       [] { int v = 0; return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, queue_kernel<false, true>, 128, 0) == cudaSuccess ? v : 1; }(),
       [] { int v = 0; return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, queue_kernel<true, true>, 128, 0) == cudaSuccess ? v : 1; }()};
   const int per_sm = std::max(1, per_sm_lod[count ? 1 : 0]);
-  const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * per_sm, (n + 127) / 128);
-  SVO_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st));
   const ClaimOrder order = claim_order(n, row);
+  const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * per_sm, (order.claims + 3) / 4);
   if (count)
-    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, ctr, viewing_distance);
+    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance);
   else
-    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, ctr, viewing_distance);
+    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance);
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }

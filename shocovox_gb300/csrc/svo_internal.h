@@ -61,6 +61,8 @@ struct SceneView {
   uint32_t mips;    // MIP maps enabled (get_by_ray_at_lod reads node MIPs)
   float mip_top;    // log2(size / D): the MIP level the LOD cast starts at (an integer)
   const DevNode* top;  // the top table (breadth-first Internal nodes of depth < kMaxStageDepth)
+  const uint4* heads;  // node heads (svo_unit.cuh): 8 planes of head_stride, one per direction octant
+  uint32_t head_stride;  // heads a plane holds
 };
 
 // Cast form selected by svo_set_cast_mode (0 automatic, 1 literal only).
@@ -70,6 +72,7 @@ struct CastQueues;  // work counters of the queued cast (svo_device.cu)
 
 struct DeviceImage {
   DevNode* nodes = nullptr;
+  uint4* heads = nullptr;  // the node heads (8 planes of node_cap), in the nodes' (or the block's) allocation
   uint32_t* voxels = nullptr;
   uint32_t* vbits = nullptr;
   uint32_t* colors = nullptr;

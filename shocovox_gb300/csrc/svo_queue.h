@@ -1,11 +1,10 @@
 // svo_queue.h -- the per-stream work counters of a scene, shared by the queued cast
 // (svo_device.cu) and the fused render (svo_render.cu).
 //
-// A queued kernel's warps claim work from a counter that starts at 0.  Launches on one stream run
-// one after another, so a stream can reuse its counter (zeroed on the stream before each launch);
-// launches on different streams may overlap, so every stream that uses the scene gets a counter
-// of its own.  The zeroing and the launch are enqueued together under the mutex, so two host
-// threads sharing a stream cannot interleave them.
+// A queued kernel's warps claim work from a counter that starts at 0 and that the launch's last warp
+// zeroes again (queue_done, svo_cast.cuh), so a launch needs nothing before it.  Launches on one
+// stream run one after another, so a stream can reuse its counter; launches on different streams
+// may overlap, so every stream that uses the scene gets a counter of its own.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -22,7 +21,7 @@ struct CastQueues {
   std::mutex m;
   cudaStream_t streams[kQueueSlots] = {};
   uint32_t used = 0;
-  unsigned long long* counters = nullptr;  // kQueueSlots device words
+  unsigned long long* counters = nullptr;  // per slot: claims taken past the warps' own, warps finished
   int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0;
 };
 
@@ -37,7 +36,7 @@ inline unsigned long long* queue_counter(CastQueues* q, cudaStream_t st) {
     if (q->used == kQueueSlots) return nullptr;
     q->streams[q->used++] = st;
   }
-  return q->counters + slot;
+  return q->counters + 2 * slot;
 }
 
 }  // namespace svo

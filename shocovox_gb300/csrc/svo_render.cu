@@ -80,12 +80,12 @@ __device__ __forceinline__ bool shade_pixel(const SceneView& s, const ViewFrame&
 }
 
 // One pixel of the example's loop; returns true where the example would panic or loop forever.
-__device__ __forceinline__ bool render_pixel(const SceneView& s, const SharedLuts& L, const ViewFrame& f, uint32_t W,
+__device__ __forceinline__ bool render_pixel(const SceneView& s, const ViewFrame& f, uint32_t W,
                                              uint32_t H, uint32_t x, uint32_t y, uchar4* __restrict__ out) {
   float dx, dy, dz;
   pixel_ray(f, x, y, dx, dy, dz);
   HitRecord h;
-  cast_one<false>(s, L, f.ox, f.oy, f.oz, dx, dy, dz, h);
+  cast_one<false>(s, kLuts, f.ox, f.oy, f.oz, dx, dy, dz, h);
   return shade_pixel(s, f, W, H, x, y, h, out);
 }
 
@@ -105,26 +105,27 @@ struct WaitingPixels {
 };
 
 __global__ void __launch_bounds__(128, 7)
-    render_queue_kernel(SceneView s, ViewFrames fs, uint32_t W, uint32_t H, uchar4* __restrict__ out,
-                        unsigned long long* __restrict__ unshaded, unsigned long long* __restrict__ counter,
+    render_queue_kernel(const __grid_constant__ SceneView s, const __grid_constant__ ViewFrames fs, uint32_t W, uint32_t H, uchar4* __restrict__ out,
+                        unsigned long long* __restrict__ unshaded, unsigned long long* __restrict__ queue,
                         uint32_t tiles_x, uint32_t tiles_per_view, uint32_t tiles) {
-  __shared__ SharedLuts L;
   __shared__ WaitingPixels waiting[4];
-  fill_shared_luts(L);
-  __syncthreads();
   const uint32_t lane = threadIdx.x & 31u;
   WaitingPixels& w = waiting[threadIdx.x >> 5];
   const size_t frame = (size_t)W * H;
+  const uint64_t warps = (uint64_t)gridDim.x * 4u;
   uint32_t count = 0;  // pixels waiting (the same in every lane)
-  bool more = true;    // tiles left
+  unsigned long long t = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
+  bool own = true, more = true;  // the warp's own tile is to take; tiles left
   for (;;) {
     bool have = false, fast = false;
     uint32_t x = 0, y = 0, target = 0, view = 0;
     float dx = 0.0f, dy = 0.0f, dz = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
     while (more && count < 32) {
-      unsigned long long t = 0;
-      if (lane == 0) t = atomicAdd(counter, 1ull);
-      t = __shfl_sync(0xFFFFFFFFu, t, 0);
+      if (!own) {
+        if (lane == 0) t = atomicAdd(queue, 1ull) + warps;
+        t = __shfl_sync(0xFFFFFFFFu, t, 0);
+      }
+      own = false;
       if (t >= tiles) {
         more = false;
         break;
@@ -189,24 +190,22 @@ __global__ void __launch_bounds__(128, 7)
     if (have) {
       const ViewFrame& f = fs.f[view];
       HitRecord h;
-      cast_entered<false>(s, L, f.ox, f.oy, f.oz, dx, dy, dz, fast, px, py, pz, target, h);
+      cast_entered<false>(s, kLuts, f.ox, f.oy, f.oz, dx, dy, dz, fast, px, py, pz, target, h);
       bad = shade_pixel(s, f, W, H, x, y, h, out + view * frame);
     }
     count_unshaded(bad, unshaded);
   }
+  queue_done(queue, warps);
 }
 
 // One 16 x 8 tile per block (8 x 4 per warp), blockIdx.z the view, for streams without a work counter.
 __global__ void __launch_bounds__(128, 7)
-    render_grid_kernel(SceneView s, ViewFrames fs, uint32_t W, uint32_t H, uchar4* __restrict__ out,
+    render_grid_kernel(const __grid_constant__ SceneView s, const __grid_constant__ ViewFrames fs, uint32_t W, uint32_t H, uchar4* __restrict__ out,
                        unsigned long long* __restrict__ unshaded) {
-  __shared__ SharedLuts L;
-  fill_shared_luts(L);
-  __syncthreads();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t x = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
   const uint32_t y = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);
-  const bool bad = x < W && y < H && render_pixel(s, L, fs.f[blockIdx.z], W, H, x, y, out + (size_t)blockIdx.z * W * H);
+  const bool bad = x < W && y < H && render_pixel(s, fs.f[blockIdx.z], W, H, x, y, out + (size_t)blockIdx.z * W * H);
   count_unshaded(bad, unshaded);
 }
 
@@ -263,7 +262,6 @@ svo_status render_views(svo_scene* sc, const svo_viewport* vps, uint32_t n_views
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, render_queue_kernel, 128, 0) == cudaSuccess ? v : 1;
       }();
       const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per_sm, 1), (tiles + 3) / 4);
-      SVO_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st));
       render_queue_kernel<<<(unsigned)grid, 128, 0, st>>>(scene_view(sc), fs, W, H, out, unshaded, ctr, (W + 7) / 8,
                                                            (uint32_t)tiles_per_view, (uint32_t)tiles);
       SVO_CUDA_TRY(cudaGetLastError());
