@@ -328,7 +328,7 @@ svo_status svo_cast_batched(svo_batch_workspace* ws, const svo_batch_item* items
  * device memory when they cast (a fixed memory budget handed over at start-up,
  * or a frame loop where a cudaMalloc would synchronise the device).  No
  * counterpart in the reference.  The item table and work counter live in one
- * scratch array compiled into the library (49,408 bytes, reserved on every GPU
+ * scratch array compiled into the library (50,432 bytes, reserved on every GPU
  * that loads the library until the process exits), so at most 128 items are
  * accepted per call; more return SVO_ERR_ARGUMENT.  The first call on a device
  * looks up the array's device address on the current device, which must be the

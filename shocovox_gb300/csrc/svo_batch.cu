@@ -960,7 +960,7 @@ constexpr uint32_t kNoAllocMaxItems = 128;  // items per call
 constexpr size_t kNoAllocTableBytes = kNoAllocMaxItems * sizeof(svo::BatchItemDev);
 constexpr size_t kNoAllocCounterOffset = (kNoAllocTableBytes + 255) / 256 * 256;
 constexpr size_t kNoAllocBytes = kNoAllocCounterOffset + 256;
-static_assert(kNoAllocBytes == 49408, "include/svo.h documents the scratch array's size");
+static_assert(kNoAllocBytes == 50432, "include/svo.h documents the scratch array's size");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 namespace {

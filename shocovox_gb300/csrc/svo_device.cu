@@ -14,10 +14,9 @@
 #include <unordered_map>
 
 #include "svo_cast.cuh"
+#include "svo_flow.cuh"
 #include "svo_queue.h"
-#include "svo_refill.cuh"
 #include "svo_trace.h"
-#include "svo_unit.cuh"
 
 namespace svo {
 
@@ -209,115 +208,37 @@ __global__ void __launch_bounds__(128, 7)
   }
 }
 
-// Refilling cast: the work queue of queue_kernel, where a warp also parks its rays at a node visit
-// once fewer than park_below of them are in flight, hands its idle lanes new entering rays from its
-// waiting list (refilled from the work counter) and resumes all of them together.  Rays in no
-// particular order then keep the lanes busy where a warp would otherwise run its few longest rays
-// alone; park_below = 0 never parks (each warp's rays run to their end, as in queue_kernel).
-template <bool kCount, bool kStage = false>
-__global__ void __launch_bounds__(128, 7)
-    refill_kernel(SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                  unsigned long long* __restrict__ queue, uint32_t park_below, uint32_t stage_n = 0) {
-  __shared__ SharedLuts L;
-  __shared__ WaitingRays waiting[4];
-  __shared__ uint32_t in_flight[4];  // rays of each warp in flight (parked ones included)
-  // each thread's ray between two runs: 23 words a thread, an odd stride, so the 32 lanes of a warp
-  // touch 32 different banks; registers hold the state only while the ray runs
-  __shared__ FastState parked[128];
-  extern __shared__ uint4 staged_smem[];
-  DevNode* stg = reinterpret_cast<DevNode*>(staged_smem);
-  fill_shared_luts(L);
-  if (kStage) stage_records(stg, s.top, stage_n);
-  __syncthreads();
+// A large batch without a row layout: a camera's rays in raster order, which queue_cast casts, or rays in
+// no order, which flow_cast casts but for those of the general forms.  The rays themselves tell (rays_mixed).
+struct FlowBlock {
+  FlowShared sh;
+  FlowLists<RayId> lists[4];
+};
+// 6 blocks per SM (80 registers): at 7 both casts' loops spill, and a camera's 925 K rays on 256^3 take 256 us
+// instead of 241 (243 in queue_kernel's own launch), 2^22 random rays on 512^3 642 us instead of 679.
+__global__ void __launch_bounds__(128, 6)
+    plain_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ queue, uint32_t refill,
+                 bool test) {
+  __shared__ union U {
+    FlowBlock flow;
+    WaitingRays waiting[4];
+    __device__ U() {}
+  } m;
+  if (test && !rays_mixed(src.rays, src.n, src.s)) {
+    queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
+    return;
+  }
   const uint32_t lane = threadIdx.x & 31u;
-  WaitingRays& w = waiting[threadIdx.x >> 5];
-  volatile uint32_t* live = in_flight + (threadIdx.x >> 5);
-  uint32_t count = 0;  // rays waiting (the same in every lane)
-  bool more = true;    // claims left
-  uint32_t park = park_below;
-  bool alive = false;
-  uint64_t i = 0;
-  for (;;) {
-    const unsigned idle = __ballot_sync(0xFFFFFFFFu, !alive);
-    const uint32_t need = __popc(idle);
-    if (need) {
-      // claims until `need` entering rays wait or no claims are left (misses written at once)
-      while (more && count < need) {
-        unsigned long long c = 0;
-        if (lane == 0) c = atomicAdd(queue, 1ull);
-        c = __shfl_sync(0xFFFFFFFFu, c, 0);
-        if (c >= order.claims) {
-          more = false;
-          break;
-        }
-        const uint64_t j = claimed_ray(order, c, lane, n);
-        bool enters = false, fast = false;
-        float px = 0.0f, py = 0.0f, pz = 0.0f;
-        uint32_t target = 0;
-        if (j < n) {
-          const float ox = __ldg(rays.ox + j), oy = __ldg(rays.oy + j), oz = __ldg(rays.oz + j);
-          const float dx = __ldg(rays.dx + j), dy = __ldg(rays.dy + j), dz = __ldg(rays.dz + j);
-          fast = !s.literal && !isnan(dx) && !isnan(dy) && !isnan(dz);
-          enters = !fast || fast_entry(s, ox, oy, oz, dx, dy, dz, px, py, pz, target);
-          if (!enters) {
-            HitRecord m;
-            miss_record(m);
-            write_hit(s, out, j, m);
-            if (kCount) write_counters(out, j, m);
-          }
-        }
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, enters);
-        if (enters) {
-          const uint32_t k = count + __popc(m & ((1u << lane) - 1u));
-          w.p[0][k] = px;
-          w.p[1][k] = py;
-          w.p[2][k] = pz;
-          w.target[k] = target | (fast ? 0x80000000u : 0u);
-          w.i[k] = j;
-        }
-        count += __popc(m);
-        __syncwarp();
-      }
-      // the k-th idle lane takes the k-th of the last `take` waiting rays
-      const uint32_t take = count < need ? count : need;
-      if (!alive) {
-        const uint32_t k = __popc(idle & ((1u << lane) - 1u));
-        if (k < take) {
-          const uint32_t at = count - take + k;
-          i = w.i[at];
-          const uint32_t tg = w.target[at];
-          const float px = w.p[0][at], py = w.p[1][at], pz = w.p[2][at];
-          const float ox = __ldg(rays.ox + i), oy = __ldg(rays.oy + i), oz = __ldg(rays.oz + i);
-          const float dx = __ldg(rays.dx + i), dy = __ldg(rays.dy + i), dz = __ldg(rays.dz + i);
-          if ((tg >> 31) == 0u) {  // a NaN direction (or literal mode): the literal form, in one go
-            HitRecord h;
-            cast_ray_literal<kCount>(s, L, ox, oy, oz, dx, dy, dz, h);
-            write_hit(s, out, i, h);
-            if (kCount) write_counters(out, i, h);
-          } else {
-            fast_start(parked[threadIdx.x], dx, dy, dz, px, py, pz, tg & 0x7FFFFFFFu);
-            alive = true;
-          }
-        }
-      }
-      count -= take;
-      if (take == 0 && !more) park = 0;  // nothing left to hand out: rays in flight run to their end
-      __syncwarp();
-      const unsigned now = __ballot_sync(0xFFFFFFFFu, alive);
-      if (lane == 0) *live = __popc(now);
-      __syncwarp();
-      if (now == 0) {
-        if (!more && count == 0) break;
-        continue;
-      }
-    }
-    if (alive) {
+  FlowLists<RayId>& lists = m.flow.lists[threadIdx.x >> 5];
+  unsigned long long c = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
+  while (uint32_t others = flow_cast(src, src.order.claims, refill, queue, c, m.flow.sh, lists)) {
+    for (uint32_t k = lane; k < others; k += 32u) {
+      const RayId id = lists.other[k];
+      float o[3], d[3];
+      src.ray(id, o, d);
       HitRecord h;
-      if (fast_run<kCount, kStage>(parked + threadIdx.x, s, L, h, live, park, stg, stage_n)) {
-        write_hit(s, out, i, h);
-        if (kCount) write_counters(out, i, h);
-        alive = false;
-      }
+      cast_one<false>(src.s, kLuts, o[0], o[1], o[2], d[0], d[1], d[2], h);
+      src.put(id, h);
     }
     __syncwarp();
   }
@@ -418,6 +339,9 @@ __global__ void __launch_bounds__(128, 7)
 constexpr uint64_t kQueueMinRays = 1u << 17;
 // The same line where the rays are read from host memory: the queue's 16 x 2 blocks read it in longer pieces.
 constexpr uint64_t kInPlaceMinRays = 1u << 15;
+// Below this many rays, of which a fifth may enter the octree, too few are left per warp for flow_cast: random rays
+// on 256^3 take 125 us instead of 117 at 320,000, 164 instead of 166 at 640,000, 216 instead of 243 at 1,280,000.
+constexpr uint64_t kFlowMinRays = 1u << 19;
 
 void destroy_queues(DeviceImage& d) {
   if (!d.queues) return;
@@ -435,6 +359,7 @@ svo_status create_queues(DeviceImage& d, cudaStream_t st) {
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm, queue_kernel<false>, 128, 0);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_count, queue_kernel<true>, 128, 0);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_plain, plain_kernel, 128, 0);
   if (e == cudaSuccess) e = cudaMalloc(&q->counters, 2 * kQueueSlots * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemsetAsync(q->counters, 0, 2 * kQueueSlots * sizeof(unsigned long long), st);
   if (e != cudaSuccess) {
@@ -519,6 +444,11 @@ SceneView scene_view(const svo_scene* sc) {
   v.top = d.top;
   v.heads = d.heads;
   v.head_stride = (uint32_t)d.node_cap;
+  v.dim_log = 0;
+  while ((v.dim >> v.dim_log) > 1u) ++v.dim_log;
+  // the unit form packs voxel coordinates in 10 bits, indexes all heads with 32 and counts cells in 23
+  v.visit_limit = v.dim <= 512u && sc->tree.size <= 65536u && d.node_cap < (1ull << 29)
+                      ? kWorkCap / work_per_visit(v.dim) : 0u;
   return v;
 }
 
@@ -993,17 +923,14 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
       // two blocks per claim halve the units of work: only where every resident warp gets at least four
       // of them (a small batch keeps the per-block claims, whose tail is shorter)
       const uint64_t warps = resident * (block / 32);
+      // rays without a row layout may go their own ways, which plain_kernel tells, where its form can take the scene
+      const bool flow = !count && v.visit_limit > 0 && !v.literal;
+      const uint64_t plain_grid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(1, q->blocks_per_sm_plain), (order.claims + 3) / 4);
       if (in_place && !count && stage_n == 0 && g_refill_below == 0 && g_pair_rows && n >= warps * 64 * 4) {
         pair_rows_kernel<<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
-      } else if (g_refill_below > 0) {
-        const size_t smem = (size_t)stage_n * sizeof(DevNode);
-        auto kern = stage_n ? (count ? refill_kernel<true, true> : refill_kernel<false, true>)
-                            : (count ? refill_kernel<true> : refill_kernel<false>);
-        SVO_CUDA_TRY(allow_dynamic_smem(kern, smem));
-        int per = 0;
-        SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));
-        const uint64_t rgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (order.claims + 3) / 4);
-        kern<<<(unsigned)rgrid, block, smem, st>>>(v, rv, hv, n, order, queue, (uint32_t)g_refill_below, stage_n);
+      } else if (flow && g_refill_below > 0) {
+        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue,
+                                                             33u - (uint32_t)g_refill_below, false);
       } else if (stage_n) {
         // the staged records take dynamic shared memory: resident blocks from this launch's size
         const size_t smem = (size_t)stage_n * sizeof(DevNode);
@@ -1015,8 +942,10 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n);
       } else if (count) {
         queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
-      } else {
+      } else if (row || in_place || !flow || n < kFlowMinRays) {
         queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
+      } else {
+        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, true);
       }
       SVO_CUDA_TRY(cudaGetLastError());
       return SVO_OK;

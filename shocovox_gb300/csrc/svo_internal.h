@@ -63,6 +63,8 @@ struct SceneView {
   const DevNode* top;  // the top table (breadth-first Internal nodes of depth < kMaxStageDepth)
   const uint4* heads;  // node heads (svo_unit.cuh): 8 planes of head_stride, one per direction octant
   uint32_t head_stride;  // heads a plane holds
+  uint32_t dim_log;      // log2(D)
+  uint32_t visit_limit;  // visits after which the unit-direction form gives a ray up (0: it takes none)
 };
 
 // Cast form selected by svo_set_cast_mode (0 automatic, 1 literal only).

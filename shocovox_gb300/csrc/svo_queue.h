@@ -22,7 +22,7 @@ struct CastQueues {
   cudaStream_t streams[kQueueSlots] = {};
   uint32_t used = 0;
   unsigned long long* counters = nullptr;  // per slot: claims taken past the warps' own, warps finished
-  int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0;
+  int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0, blocks_per_sm_plain = 0;
 };
 
 // The counter of stream `st` (claimed on first use), or nullptr when the scene has none for it:
