@@ -900,6 +900,22 @@ uint32_t grid_lanes(uint64_t n) {
   return lanes;
 }
 
+}  // namespace
+// plain_kernel over one batch whose rays are in no order (svo_batch.cu).  `queue`: two device words, zero.
+svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView& hits, uint64_t n, uint32_t refill,
+                        uint32_t blocks_per_sm, unsigned long long* queue, cudaStream_t st) {
+  int dev = 0, sms = 0, per = (int)blocks_per_sm;
+  SVO_CUDA_TRY(cudaGetDevice(&dev));
+  SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (per == 0) SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, plain_kernel, 128, 0));
+  const ClaimOrder order = claim_order(n, 0);
+  const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)std::max(per, 1), (order.claims + 3) / 4);
+  plain_kernel<<<(unsigned)grid, 128, 0, st>>>(ArraySource{v, rays, hits, n, order}, queue, refill, false);
+  SVO_CUDA_TRY(cudaGetLastError());
+  return SVO_OK;
+}
+namespace {
+
 // `in_place`: rays and hits are host memory the device reads and writes through the CPU's page
 // tables; the claims are then 16 x 2 blocks (two 64-byte pieces of each array per warp instead of
 // four 32-byte ones), which the host link serves faster than 8 x 4 blocks.

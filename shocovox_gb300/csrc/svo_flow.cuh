@@ -469,6 +469,9 @@ struct ArraySource {
   __device__ __forceinline__ void put(const RayId& id, HitRecord& h) const { write_hit(s, out, id.i, h); }
 };
 
+svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView& hits, uint64_t n, uint32_t refill,
+                        uint32_t blocks_per_sm, unsigned long long* queue, cudaStream_t st);
+
 // Whether neighbouring rays of a batch go their own ways: of 32 pairs of rays 16 apart, spread over the batch,
 // fewer than 24 head into one octant, within 25 degrees, from origins within an eighth of the octree; and all are
 // of the unit form.  Every warp of a launch reads the same 12 x 32 values and comes to the same answer.

@@ -139,7 +139,7 @@ SVO_UHD bool unit_eligible(const SceneView& s, float ox, float oy, float oz, flo
   const float len2 = (dx * dx + dy * dy) + dz * dz;
   const float far = s.size * 1024.0f;
   auto same = [](float d) { return (1.0f + d >= 1.0f) == !signbit(d); };
-  return !s.literal && fabsf(len2 - 1.0f) <= 0x1p-12f && fabsf(ox) <= far && fabsf(oy) <= far && fabsf(oz) <= far &&
+  return !s.literal && s.visit_limit != 0u && fabsf(len2 - 1.0f) <= 0x1p-12f && fabsf(ox) <= far && fabsf(oy) <= far && fabsf(oz) <= far &&
          same(dx) && same(dy) && same(dz);
 }
 
