@@ -99,7 +99,7 @@ constexpr uint32_t kBatchMaxBlock = 128;
 
 // Rays that miss their octree's root box get their miss written at once; the entering rays of a
 // partly entering round of 32 indices wait in the warp's slice of shared memory (their index, item,
-// the point where they enter and its octant) until 32 of them fill the warp; their origin and
+// the point where they enter and its octant) until `pack` of them (pack_target) are there; their origin and
 // direction are read again when they are cast (less shared memory per block leaves more L1).
 struct WaitingBatchRays {
   float p[3][64];
@@ -111,7 +111,7 @@ struct WaitingBatchRays {
 template <bool kCount, bool kStage = false>
 __global__ void __launch_bounds__(kBatchMaxBlock, 7)
     batched_kernel(const BatchItemDev* __restrict__ items, uint32_t n_items, uint64_t total,
-                   unsigned long long* __restrict__ counter, uint32_t chunk) {
+                   unsigned long long* __restrict__ counter, uint32_t chunk, uint32_t pack) {
   __shared__ uint64_t s_begin[kMaxSharedItems];
   __shared__ WaitingBatchRays waiting[kBatchMaxBlock / 32];
   extern __shared__ uint4 staged_smem[];
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 7)
     uint64_t i = 0;
     uint32_t item = 0, target = 0;
     float ox = 0.0f, oy = 0.0f, oz = 0.0f, dx = 0.0f, dy = 0.0f, dz = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
-    while (count < 32) {
+    while (count < pack) {
       if (next >= chunk) {
         if (!more) break;
         if (lane == 0) base = atomicAdd(counter, (unsigned long long)chunk);
@@ -337,7 +337,8 @@ svo_status launch_claimed(const BatchItemDev* d_items, uint32_t n_items, uint64_
   grid = std::min<uint64_t>(grid, (warps_needed * 32 + block - 1) / block);
   grid = std::max<uint64_t>(grid, 1);
   SVO_CUDA_TRY(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st));
-  kern<<<(unsigned)grid, block, smem, st>>>(d_items, n_items, total, d_counter, chunk);
+  kern<<<(unsigned)grid, block, smem, st>>>(d_items, n_items, total, d_counter, chunk,
+                                            pack_target(total / 32, (uint64_t)sm_count * per_sm * (block / 32)));
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128, 7)
 //
 // Rays that miss the octree's root box get their miss written at once.  A claim whose rays all
 // enter is cast as it is; the entering rays of other claims wait in the warp's slice of shared
-// memory, with the point where they enter, until 32 of them fill the warp, so that rays from
+// memory, with the point where they enter, until `pack` of them (pack_target) are there, so that rays from
 // outside the octree (most of them missing it) do not leave most lanes idle.
 struct WaitingRays {  // the ray's origin and direction are read again from the ray arrays
   float p[3][64];
@@ -105,7 +105,7 @@ template <bool kCount, bool kLod = false, bool kStage = false>
 __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& rays, const HitsView& out, uint64_t n,
                                            const ClaimOrder& order, unsigned long long* __restrict__ queue,
                                            const SharedLuts& L, WaitingRays (&waiting)[4], const DevNode* stg,
-                                           float viewing_distance = 0.0f, uint32_t stage_n = 0) {
+                                           float viewing_distance = 0.0f, uint32_t stage_n = 0, uint32_t pack = 32u) {
   const uint32_t lane = threadIdx.x & 31u;
   WaitingRays& w = waiting[threadIdx.x >> 5];
   uint32_t count = 0;  // rays waiting (the same in every lane)
@@ -115,7 +115,7 @@ __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& r
     uint64_t i = 0;
     float ox = 0.0f, oy = 0.0f, oz = 0.0f, dx = 0.0f, dy = 0.0f, dz = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
     uint32_t target = 0;
-    while (more && count < 32) {
+    while (more && count < pack) {
       unsigned long long c = 0;
       if (lane == 0) c = atomicAdd(queue, 1ull);
       c = __shfl_sync(0xFFFFFFFFu, c, 0);
@@ -193,7 +193,7 @@ __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& r
 template <bool kCount, bool kLod = false, bool kStage = false>
 __global__ void __launch_bounds__(128, 7)
     queue_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                 unsigned long long* __restrict__ queue, float viewing_distance = 0.0f, uint32_t stage_n = 0) {
+                 unsigned long long* __restrict__ queue, float viewing_distance, uint32_t stage_n, uint32_t pack) {
   __shared__ WaitingRays waiting[4];
   if constexpr (kStage) {
     __shared__ SharedLuts L;
@@ -202,9 +202,9 @@ __global__ void __launch_bounds__(128, 7)
     fill_shared_luts(L);
     stage_records(stg, s.top, stage_n);
     __syncthreads();
-    queue_cast<kCount, kLod, kStage>(s, rays, out, n, order, queue, L, waiting, stg, viewing_distance, stage_n);
+    queue_cast<kCount, kLod, kStage>(s, rays, out, n, order, queue, L, waiting, stg, viewing_distance, stage_n, pack);
   } else {
-    queue_cast<kCount, kLod>(s, rays, out, n, order, queue, kLuts, waiting, nullptr, viewing_distance);
+    queue_cast<kCount, kLod>(s, rays, out, n, order, queue, kLuts, waiting, nullptr, viewing_distance, 0, pack);
   }
 }
 
@@ -939,6 +939,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
       // two blocks per claim halve the units of work: only where every resident warp gets at least four
       // of them (a small batch keeps the per-block claims, whose tail is shorter)
       const uint64_t warps = resident * (block / 32);
+      const uint32_t pack = pack_target(order.claims, warps);
       // rays without a row layout may go their own ways, which plain_kernel tells, where its form can take the scene
       const bool flow = !count && v.visit_limit > 0 && !v.literal;
       const uint64_t plain_grid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(1, q->blocks_per_sm_plain), (order.claims + 3) / 4);
@@ -955,11 +956,11 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         int per = 0;
         SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));
         const uint64_t sgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (order.claims + 3) / 4);
-        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n);
+        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n, pack);
       } else if (count) {
-        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
+        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack);
       } else if (row || in_place || !flow || n < kFlowMinRays) {
-        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
+        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack);
       } else {
         plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, true);
       }
@@ -1234,10 +1235,11 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
   const int per_sm = std::max(1, per_sm_lod[count ? 1 : 0]);
   const ClaimOrder order = claim_order(n, row);
   const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * per_sm, (order.claims + 3) / 4);
+  const uint32_t pack = pack_target(order.claims, (uint64_t)q->sm_count * per_sm * 4u);
   if (count)
-    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance);
+    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance, 0, pack);
   else
-    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance);
+    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance, 0, pack);
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }

@@ -96,8 +96,8 @@ __device__ __forceinline__ void count_unshaded(bool bad, unsigned long long* uns
 
 // Warps claim 8 x 4 pixel tiles (row-major over the image) from the stream's work counter.  Pixels
 // whose ray misses the root box are coloured at once; the entering rays of a tile that has some
-// wait in the warp's slice of shared memory (direction, entry point, pixel) until 32 of them fill
-// the warp, so that sky pixels do not leave lanes idle.
+// wait in the warp's slice of shared memory (direction, entry point, pixel) until `pack` of them
+// (pack_target) are there, so that sky pixels do not leave lanes idle.
 struct WaitingPixels {
   float d[3][64], p[3][64];
   uint32_t target[64];  // octant of the entry point | view << 8; bit 31: fast form
@@ -107,7 +107,7 @@ struct WaitingPixels {
 __global__ void __launch_bounds__(128, 7)
     render_queue_kernel(const __grid_constant__ SceneView s, const __grid_constant__ ViewFrames fs, uint32_t W, uint32_t H, uchar4* __restrict__ out,
                         unsigned long long* __restrict__ unshaded, unsigned long long* __restrict__ queue,
-                        uint32_t tiles_x, uint32_t tiles_per_view, uint32_t tiles) {
+                        uint32_t tiles_x, uint32_t tiles_per_view, uint32_t tiles, uint32_t pack) {
   __shared__ WaitingPixels waiting[4];
   const uint32_t lane = threadIdx.x & 31u;
   WaitingPixels& w = waiting[threadIdx.x >> 5];
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(128, 7)
     bool have = false, fast = false;
     uint32_t x = 0, y = 0, target = 0, view = 0;
     float dx = 0.0f, dy = 0.0f, dz = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
-    while (more && count < 32) {
+    while (more && count < pack) {
       if (!own) {
         if (lane == 0) t = atomicAdd(queue, 1ull) + warps;
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(128, 7)
         more = false;
         break;
       }
-      view = (uint32_t)(t / tiles_per_view);
-      const uint32_t tv = (uint32_t)(t - (unsigned long long)view * tiles_per_view);
+      view = (uint32_t)t / tiles_per_view;
+      const uint32_t tv = (uint32_t)t - view * tiles_per_view;
       x = (tv % tiles_x) * 8u + (lane & 7u);
       y = (tv / tiles_x) * 4u + (lane >> 3);
       bool enters = false;
@@ -263,7 +263,8 @@ svo_status render_views(svo_scene* sc, const svo_viewport* vps, uint32_t n_views
       }();
       const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per_sm, 1), (tiles + 3) / 4);
       render_queue_kernel<<<(unsigned)grid, 128, 0, st>>>(scene_view(sc), fs, W, H, out, unshaded, ctr, (W + 7) / 8,
-                                                           (uint32_t)tiles_per_view, (uint32_t)tiles);
+                                                           (uint32_t)tiles_per_view, (uint32_t)tiles,
+                                                           pack_target(tiles, (uint64_t)q->sm_count * std::max(per_sm, 1) * 4u));
       SVO_CUDA_TRY(cudaGetLastError());
       return SVO_OK;
     }
