@@ -211,9 +211,10 @@ svo_status svo_set_device_allocator(svo_alloc_fn alloc, svo_free_fn release, voi
 
 /* ---- the hot path: Octree::get_by_ray (src/raytracing/raytracing_on_cpu.rs:316-565) ---- */
 /* n rays in device memory -> per-ray hits in device memory.  Allocates nothing.
- * Batches of 32768 rays and more run as a work queue: warps claim 32 rays at a time from a
+ * Batches of 131,072 rays and more run as a work queue: warps claim 32 rays at a time from a
  * counter that the scene keeps per stream (up to 64 streams; casts on further streams, and on
- * cudaStreamPerThread, use one thread per ray).  Casts of one scene on different streams may
+ * cudaStreamPerThread, use one thread per ray).  From 524,288 rays on, rays without a row layout that
+ * go their own ways (a sample of them is looked at on the device) are cast a step of each at a time.  Casts of one scene on different streams may
  * overlap.  A CUDA graph that captured a cast reuses the counter of the stream it was captured
  * on: do not run it concurrently with casts on that stream. */
 svo_status svo_cast(svo_scene* scene, const svo_rays* rays, uint64_t n, const svo_hits* hits, void* stream);
@@ -225,9 +226,9 @@ svo_status svo_cast_lod(svo_scene* scene, const svo_rays* rays, uint64_t n, cons
                         void* stream);
 /* Same cast with host ray and hit buffers, stream synchronised before return.  The batch is staged
  * in chunks through a per-scene device workspace that grows on demand, copies overlapping the casts
- * (with pinned host memory); camera images given with their row length (svo_cast_host_rows) are
- * read and written in place where the device reads host memory through the CPU's page tables
- * (Grace), see svo_set_host_transfer: a large image (four claims or more per resident warp) is cast
+ * (with pinned host memory); batches of fewer than 131,072 rays, and camera images given with their row
+ * length (svo_cast_host_rows), are read and written in place where the device reads host memory through
+ * the CPU's page tables (Grace), see svo_set_host_transfer: a large image (four claims or more per resident warp) is cast
  * two 16 x 2 ray blocks per warp, each hit field written row by row in 32-ray pieces. */
 svo_status svo_cast_host(svo_scene* scene, const svo_rays* rays, uint64_t n, const svo_hits* hits, void* stream);
 /* The three casts above for rays laid out as rows of row_length rays (a camera image in raster
@@ -291,33 +292,27 @@ typedef struct {
   uint32_t blocks_per_sm;  /* persistent CTAs per SM; 0 = default from occupancy */
   uint32_t block_shape;    /* rays of an item with a row length cast together: 0 or 3 = 8 x 4, 4 = 16 x 2,
                               5 = 32 x 1 (log2 of the width) */
-  uint32_t sort_key;       /* order of the rays of the items without a row length: 0 = index order;
-                              1 = sorted by (item, octant of the direction, Morton code of the point
-                              where the ray enters the octree), so that a warp's rays walk much the
-                              same nodes (svo_cast_batched only: needs the workspace's buffers, which
-                              grow to 128 bytes per such ray) */
+  uint32_t sort_key;       /* the rays of the items without a row length: 0 = cast 32 neighbours at a time,
+                              1 = in no particular order: cast a step of each ray at a time, a warp's
+                              idle lanes taking new rays (svo_cast_batched only; fewer than 2^32 such
+                              rays per call) */
   uint32_t staging_depth;  /* top tree levels staged in shared memory by every block: the Internal nodes of
                               depth < staging_depth (0..4) of each scene of the call, as far as 48 KB of
                               records per block reach (scenes past that read their nodes from L1/L2) */
-  uint32_t refill_below;   /* with sort_key 1: the sorted rays' cast parks a warp's rays at a node visit once
-                              fewer than refill_below (1..32) are in flight, gives its idle lanes the next
-                              sorted rays and resumes (see svo_set_refill); 0 = each warp's rays run to
-                              their ends.  The hits are the same for every value. */
+  uint32_t refill_below;   /* with sort_key 1: a warp gives its idle lanes new rays once fewer than
+                              refill_below (1..32) are in flight (see svo_set_refill); 0 = 21.  The hits
+                              are the same for every value. */
 } svo_launch_config;
 
 /* Casts every item's rays in one persistent kernel launch driven by a device
  * work counter.  The per-launch item table and counter live in a workspace
  * owned by `ws` (create it once; it grows only when the item count grows).
- * With sort_key 1 the items without a row length are cast through the ray sort
- * instead: a binning launch (misses written at once), a scan of the bucket
- * counts, a scatter into bucket order and a persistent cast of the sorted
- * entering rays, all on `stream`; the hits are the same as in index order.  The
- * sort's buffers grow only when the rays (or buckets) of a call outgrow them:
- * make the largest call once before a stream capture.  A graph that captured a
+ * With sort_key 1 the items without a row length are cast by a launch of their
+ * own before it; the hits are the same.  A graph that captured a
  * call reads the workspace's host-side item table and device buffers at every
  * replay: while that graph may still be replayed, make other casts through
  * another workspace (a call on this one rewrites the table the graph reads,
- * and one that outgrows the buffers frees those the graph uses). */
+ * and one of more items frees the tables the graph uses). */
 typedef struct svo_batch_workspace svo_batch_workspace;
 svo_status svo_batch_workspace_create(svo_batch_workspace** out);
 void svo_batch_workspace_destroy(svo_batch_workspace* ws);
@@ -428,8 +423,8 @@ svo_status svo_selftest_luts(uint64_t* ray_to_node, uint32_t* octant_step, uint6
  * same results; mode 1 exists so tests can check that. */
 svo_status svo_set_cast_mode(int32_t mode);
 /* How svo_cast_host moves rays and hits (process-wide): 0 (default) lets the kernel read and write
- * the host buffers in place for batches with a row layout (svo_cast_host_rows, row_length >= 16)
- * when the device accesses host memory through the CPU's page tables (Grace systems), and stages
+ * the host buffers in place for batches of fewer than 131,072 rays and for batches with a row
+ * layout (svo_cast_host_rows, row_length >= 16) when the device accesses host memory through the CPU's page tables (Grace systems), and stages
  * copies otherwise; 1 always stages copies (chunks over three streams); 2 always accesses host
  * memory directly (an error where the device cannot); 3 as 2, with each warp writing its own 16 x 2
  * ray block (pieces of 64 and 16 bytes a row) instead of two blocks' rows of 32 rays (pieces of 128
@@ -442,11 +437,11 @@ svo_status svo_set_host_transfer(int32_t mode);
  * The results are the same at every depth; the batched cast takes its depth from
  * svo_launch_config.staging_depth.  No counterpart in the reference. */
 svo_status svo_set_staging_depth(int32_t depth);
-/* Lane refill of the plain casts launched afterwards (process-wide): 0 (default) casts each warp's
- * 32 rays to their ends; 1..32: a warp whose rays in flight drop below park_below stops them at their
- * next node visit, gives its idle lanes new rays and continues all of them together, so that rays of
- * very different lengths (rays in no particular order) keep the lanes busy.  The results are the same
- * for every value.  No counterpart in the reference. */
+/* Lane refill of the plain casts launched afterwards (process-wide): 0 (default) lets large batches
+ * without a row layout choose by a sample of their rays; 1..32: every batch of 131,072 rays and more is
+ * cast a step of each ray at a time, and a warp whose rays in flight drop below park_below gives its idle
+ * lanes new rays, so that rays of very different lengths (rays in no particular order) keep the
+ * lanes busy.  The results are the same for every value.  No counterpart in the reference. */
 svo_status svo_set_refill(int32_t park_below);
 
 #ifdef __cplusplus

@@ -335,10 +335,9 @@ __global__ void __launch_bounds__(128, 7)
 }
 
 // Below this many rays one grid with fewer rays per warp (grid_lanes) is faster than the work queue: 119,860 camera
-// rays on 512^3 135 us against 157, on 256^3 117 against 120; at 160,000 the two are even.
+// rays on 512^3 135 us against 157, on 256^3 117 against 120; at 160,000 the two are even.  The same holds in host
+// memory read in place: 120,000 camera rays 149 us against 165, 130,000 random ones 503 against 604.
 constexpr uint64_t kQueueMinRays = 1u << 17;
-// The same line where the rays are read from host memory: the queue's 16 x 2 blocks read it in longer pieces.
-constexpr uint64_t kInPlaceMinRays = 1u << 15;
 // Below this many rays, of which a fifth may enter the octree, too few are left per warp for flow_cast: random rays
 // on 256^3 take 125 us instead of 117 at 320,000, 164 instead of 166 at 640,000, 216 instead of 243 at 1,280,000.
 constexpr uint64_t kFlowMinRays = 1u << 19;
@@ -928,7 +927,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
   const bool count = counts_requested(*hits);
   const unsigned block = 128;
   CastQueues* q = sc->dev.queues;
-  if (q && n >= (in_place ? kInPlaceMinRays : kQueueMinRays)) {
+  if (q && n >= kQueueMinRays) {
     std::lock_guard<std::mutex> lock(q->m);
     if (unsigned long long* queue = queue_counter(q, st)) {
       const int per_sm = std::max(1, count ? q->blocks_per_sm_count : q->blocks_per_sm);
@@ -968,7 +967,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
       return SVO_OK;
     }
   }
-  const uint32_t lanes = in_place ? 5u : grid_lanes(n);
+  const uint32_t lanes = grid_lanes(n);
   const uint64_t grid = (((n + (1u << lanes) - 1) >> lanes) + 3) / 4;
   if (grid > 0x7FFFFFFFull) return fail(SVO_ERR_ARGUMENT, "svo_cast: too many rays for one launch");
   if (count)
@@ -1261,9 +1260,11 @@ svo_status svo_cast_host_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, u
   // Where the device reads host memory through the CPU's page tables (Grace: NVLink-C2C with
   // address translation), the kernel reads the rays and writes the hits in place; elsewhere the
   // batch goes through staged copies.
-  // By default only batches with a row layout (camera images) are read in place: the work queue
-  // casts the rays that enter the octree out of order (packed into full warps), and where many rays
-  // miss the octree their hits would reach host memory in small scattered pieces.
+  // By default batches without a row layout are read in place only below the work queue's size: one
+  // grid then writes the hits in order, and the copies' calls alone (six arrays in, up to 18 out, three
+  // streams) take 130 us: one ray 50 us against 175, 20,000 rays 162 against 352, 130,000 503 against 696.  The
+  // work queue casts the rays that enter the octree out of order, and where many miss it
+  // their hits would reach host memory in small scattered pieces (250,000 rays: 1,207 against 1,132).
   int direct = 0;
   if (g_host_transfer != 1) {
     int dev = 0;
@@ -1271,7 +1272,7 @@ svo_status svo_cast_host_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, u
     SVO_CUDA_TRY(cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev));
     if (g_host_transfer == 2 && !direct)
       return fail(SVO_ERR_ARGUMENT, "svo_cast_host: this device cannot access host memory directly");
-    if (g_host_transfer == 0 && row_length < 16) direct = 0;
+    if (g_host_transfer == 0 && row_length < 16 && n >= kQueueMinRays) direct = 0;
   }
   if (!direct) return cast_host_pipelined(sc, rays, n, hits, st, row_length);
   const svo_status rc = launch_cast(sc, rays, n, hits, st, row_length, true);

@@ -73,3 +73,18 @@ def test_heads_follow_in_place_syncs(oracle_mod):
                 t.clear(pos) if k == 1 else t.insert(pos, 0x11223344 + k, 7)
         p.sync()
         assert_same_hits(p.cast_host(origins, dirs, fields=UNCOUNTED), o.cast(origins, dirs, threads=8), label="sync %d" % k)
+
+
+@pytest.mark.parametrize("n", [1, 33, 4097, GRID - 1, GRID])
+def test_host_buffers_in_place_and_staged(oracle_mod, n):
+    rng = np.random.default_rng(n)
+    o, p = both(oracle_mod, 64, 4, svo.gen_scene(3, 64, 4, seed=8, occupancy=0.1, spheres=2))
+    origins, dirs = random_rays(rng, 64, n)
+    ref = o.cast(origins, dirs, threads=16)
+    for mode in (0, 1):  # the default, staged copies
+        svo.check(svo.lib().svo_set_host_transfer(mode))
+        try:
+            assert_same_hits(p.cast_host(origins, dirs), ref, counters=True, label="mode %d" % mode)
+            assert_same_hits(p.cast_host(origins, dirs, fields=UNCOUNTED), ref, label="uncounted, mode %d" % mode)
+        finally:
+            svo.check(svo.lib().svo_set_host_transfer(0))
