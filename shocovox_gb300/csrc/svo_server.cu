@@ -14,6 +14,9 @@
 // work already running.
 #include <cuda_runtime.h>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -48,11 +51,26 @@ struct CamParams {
   uint32_t width, height;
 };
 
-// The per-pixel part of svo_gen_camera_rays, same operations in the same order.
-__global__ void camera_rays_kernel(CamParams c, float* ox, float* oy, float* oz, float* dx, float* dy, float* dz) {
+// The cameras of one launch (kernel parameters), blockIdx.y's each.
+constexpr uint32_t kCameras = 32;
+struct CamJobs {
+  CamParams c[kCameras];
+  float* rays[kCameras];  // six arrays, `pitch` floats apart
+  uint64_t pitch[kCameras];
+};
+
+// The per-pixel part of svo_gen_camera_rays, same operations in the same order.  Bound by the 24 bytes
+// a ray that it writes; one launch for all requests of a batch (24 of them: 156 us in launches of
+// their own, 101 together).
+__global__ void __launch_bounds__(256) camera_rays_kernel(const __grid_constant__ CamJobs jobs) {
+  const CamParams& c = jobs.c[blockIdx.y];
+  float *const ox = jobs.rays[blockIdx.y], *const oy = ox + jobs.pitch[blockIdx.y], *const oz = oy + jobs.pitch[blockIdx.y];
+  float *const dx = oz + jobs.pitch[blockIdx.y], *const dy = dx + jobs.pitch[blockIdx.y], *const dz = dy + jobs.pitch[blockIdx.y];
   const uint64_t n = (uint64_t)c.width * c.height;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t px = (uint32_t)(i % c.width), py = (uint32_t)(i / c.width);
+    // a 64-bit division is a long sequence: only images past 32 bits take it
+    const uint32_t py = (n >> 32) ? (uint32_t)(i / c.width) : (uint32_t)i / c.width;
+    const uint32_t px = (uint32_t)(i - (uint64_t)py * c.width);
     const float u = (2.0f * ((float)px + 0.5f) / (float)c.width - 1.0f) * c.tan_half * c.aspect;
     const float v = (1.0f - 2.0f * ((float)py + 0.5f) / (float)c.height) * c.tan_half;
     // add(add(fwd, mul(right, u)), mul(up, v)) with up = (0, 1, 0)
@@ -66,6 +84,44 @@ __global__ void camera_rays_kernel(CamParams c, float* ox, float* oy, float* oz,
     dy[i] = vy / l;
     dz[i] = vz / l;
   }
+}
+
+// Device memory into host memory that the device writes through the CPU's page tables: pieces of a launch's results,
+// blockIdx.y's each.  Bound by the link.  cudaMemcpyAsync into pageable memory returns only when
+// the copy is done, one field of one request at a time, so nothing overlapped it.
+constexpr uint32_t kCopies = 128;
+struct CopyJobs {
+  const char* src[kCopies];  // 256-byte aligned
+  char* dst[kCopies];
+  uint64_t bytes[kCopies];
+};
+__global__ void __launch_bounds__(256) copy_out_kernel(const __grid_constant__ CopyJobs jobs) {
+  const char* src = jobs.src[blockIdx.y];
+  char* dst = jobs.dst[blockIdx.y];
+  const uint64_t bytes = jobs.bytes[blockIdx.y], at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t align = reinterpret_cast<uintptr_t>(dst) & 15u;
+  uint64_t done = 0;  // copied in wide pieces by all blocks together
+  if (align == 0) {
+    for (uint64_t k = at; k < bytes / 16; k += step) reinterpret_cast<uint4*>(dst)[k] = __ldcs(reinterpret_cast<const uint4*>(src) + k);
+    done = bytes / 16 * 16;
+  } else if (align % 4 == 0) {
+    for (uint64_t k = at; k < bytes / 4; k += step) reinterpret_cast<uint32_t*>(dst)[k] = __ldcs(reinterpret_cast<const uint32_t*>(src) + k);
+    done = bytes / 4 * 4;
+  }
+  for (uint64_t k = done + at; k < bytes; k += step) dst[k] = src[k];
+}
+
+// Gives the pages under a result buffer memory, contents unchanged, before the device writes them: a page that
+// the device touches first costs it a fault (24 requests into fresh buffers: 23 ms against 8).  The
+// host does it while the cast runs.  Kernels without the call leave it to the device.
+void populate(void* p, uint64_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p) / page * page, b = reinterpret_cast<uintptr_t>(p) + bytes;
+  if (bytes) madvise(reinterpret_cast<void*>(a), (b - a + page - 1) / page * page, MADV_POPULATE_WRITE);
 }
 
 double now_s() {
@@ -110,6 +166,7 @@ struct svo_server {
   static constexpr size_t kMaxScenes = 4096;  // scene slots never move: the vector is reserved once
   svo_server_config cfg{};
   int device = 0;
+  int direct = 0;  // the device writes host memory through the CPU's page tables
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
   std::deque<svo::Request*> pending;
@@ -211,6 +268,19 @@ svo_status launch(svo_server* sv, LaunchSlot& ls, size_t n_scenes, LaunchCounts&
     if (ready) SRV_CUDA(cudaStreamWaitEvent(ls.st, ready, 0));
   }
   std::vector<svo_batch_item> items(ls.reqs.size());
+  CamJobs cams;
+  uint32_t n_cams = 0;
+  uint64_t most = 0;  // rays of the largest of them
+  auto launch_cameras = [&]() -> svo_status {
+    if (n_cams) {
+      const unsigned x = (unsigned)std::min<uint64_t>((most + 255) / 256, std::max<uint64_t>(1, 8192 / n_cams));
+      camera_rays_kernel<<<dim3(x, n_cams), 256, 0, ls.st>>>(cams);
+      SRV_CUDA(cudaGetLastError());
+    }
+    n_cams = 0;
+    most = 0;
+    return SVO_OK;
+  };
   size_t o = 0;
   for (size_t i = 0; i < ls.reqs.size(); ++i) {
     Request* q = ls.reqs[i];
@@ -223,9 +293,14 @@ svo_status launch(svo_server* sv, LaunchSlot& ls, size_t n_scenes, LaunchCounts&
     camera_frame(q->r.eye, q->r.target, q->r.fov_deg, q->r.width, q->r.height, &f);
     CamParams c{q->r.eye[0], q->r.eye[1], q->r.eye[2], f.fwd[0], f.fwd[1], f.fwd[2], f.right[0], f.right[1],
                 f.right[2], f.tan_half, f.aspect, q->r.width, q->r.height};
-    const unsigned blocks = (unsigned)std::min<uint64_t>((q->n + 255) / 256, 4096);
-    camera_rays_kernel<<<blocks, 256, 0, ls.st>>>(c, r[0], r[1], r[2], r[3], r[4], r[5]);
-    SRV_CUDA(cudaGetLastError());
+    cams.c[n_cams] = c;
+    cams.rays[n_cams] = r[0];
+    cams.pitch[n_cams] = (uint64_t)(r[1] - r[0]);
+    most = std::max(most, q->n);
+    if (++n_cams == kCameras) {
+      rc = launch_cameras();
+      if (rc != SVO_OK) return rc;
+    }
     svo_batch_item& it = items[i];
     std::memset(&it, 0, sizeof(it));
     it.scene = sv->scenes[q->r.scene_id].scene;
@@ -240,15 +315,46 @@ svo_status launch(svo_server* sv, LaunchSlot& ls, size_t n_scenes, LaunchCounts&
         o += ((kHitFieldBytes[fi] * q->n + 255) / 256) * 256;
       }
   }
+  rc = launch_cameras();
+  if (rc != SVO_OK) return rc;
   rc = svo_cast_batched(ls.ws, items.data(), (uint32_t)items.size(), &sv->cfg.launch, ls.st);
   if (rc != SVO_OK) return rc;
+  CopyJobs copies;
+  uint32_t n_copies = 0;
+  uint64_t longest = 0;
+  auto launch_copies = [&]() -> svo_status {
+    if (n_copies) {
+      const unsigned x = (unsigned)std::min<uint64_t>((longest / 16 + 255) / 256 + 1, std::max<uint64_t>(1, 4096 / n_copies));
+      copy_out_kernel<<<dim3(x, n_copies), 256, 0, ls.st>>>(copies);
+      SRV_CUDA(cudaGetLastError());
+    }
+    n_copies = 0;
+    longest = 0;
+    return SVO_OK;
+  };
   for (size_t i = 0; i < ls.reqs.size(); ++i) {
     Request* q = ls.reqs[i];
     void* const* hf = reinterpret_cast<void* const*>(&q->r.hits);
     void** df = reinterpret_cast<void**>(&items[i].hits);
-    for (int f = 0; f < kHitFields; ++f)
-      if (hf[f]) SRV_CUDA(cudaMemcpyAsync(hf[f], df[f], kHitFieldBytes[f] * q->n, cudaMemcpyDeviceToHost, ls.st));
+    for (int f = 0; f < kHitFields; ++f) {
+      if (!hf[f]) continue;
+      if (!sv->direct) {
+        SRV_CUDA(cudaMemcpyAsync(hf[f], df[f], kHitFieldBytes[f] * q->n, cudaMemcpyDeviceToHost, ls.st));
+        continue;
+      }
+      populate(hf[f], kHitFieldBytes[f] * q->n);
+      copies.src[n_copies] = static_cast<const char*>(df[f]);
+      copies.dst[n_copies] = static_cast<char*>(hf[f]);
+      copies.bytes[n_copies] = kHitFieldBytes[f] * q->n;
+      longest = std::max(longest, copies.bytes[n_copies]);
+      if (++n_copies == kCopies) {
+        rc = launch_copies();
+        if (rc != SVO_OK) return rc;
+      }
+    }
   }
+  rc = launch_copies();
+  if (rc != SVO_OK) return rc;
   SRV_CUDA(cudaEventRecord(ls.done, ls.st));
   cnt.launches++;
   return SVO_OK;
@@ -372,6 +478,8 @@ svo_status svo_server_create(const svo_server_config* cfg, svo_server** out) {
   sv->cfg = c;
   sv->scenes.reserve(svo_server::kMaxScenes);
   cudaGetDevice(&sv->device);
+  if (cudaDeviceGetAttribute(&sv->direct, cudaDevAttrPageableMemoryAccessUsesHostPageTables, sv->device) != cudaSuccess)
+    sv->direct = 0;
   sv->slots.resize(c.max_inflight);
   for (LaunchSlot& ls : sv->slots) {
     cudaError_t e = cudaStreamCreateWithFlags(&ls.st, cudaStreamNonBlocking);
