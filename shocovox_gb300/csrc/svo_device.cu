@@ -1007,6 +1007,12 @@ void destroy_pipeline(DeviceImage& d) {
   d.ws_bytes = 0;
 }
 
+// The pages of large host hit fields, while a cast that will write them (or a copy that waits for it) runs.
+void populate_hits(const svo_hits* hits, uint64_t n) {
+  void* const* fields = reinterpret_cast<void* const*>(hits);
+  for (int f = 0; f < kHitFields; ++f) populate(fields[f], kHitFieldBytes[f] * n, 1u << 20);
+}
+
 svo_status cast_host_pipelined(svo_scene* sc, const svo_rays* rays, uint64_t n, const svo_hits* hits,
                                cudaStream_t caller, uint64_t row) {
   DeviceImage& d = sc->dev;
@@ -1066,6 +1072,7 @@ svo_status cast_host_pipelined(svo_scene* sc, const svo_rays* rays, uint64_t n, 
     svo_rays drays{dr[0], dr[1], dr[2], dr[3], dr[4], dr[5]};
     svo_status rc = launch_cast(sc, &drays, m, &dh, st, row);
     if (rc != SVO_OK) return rc;
+    if (off == 0) populate_hits(hits, n);
     for (int f = 0; f < kHitFields; ++f)
       if (host_fields[f])
         SVO_CUDA_TRY(cudaMemcpyAsync(static_cast<char*>(host_fields[f]) + off * kHitFieldBytes[f], dev_fields[f],
@@ -1277,6 +1284,7 @@ svo_status svo_cast_host_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, u
   if (!direct) return cast_host_pipelined(sc, rays, n, hits, st, row_length);
   const svo_status rc = launch_cast(sc, rays, n, hits, st, row_length, true);
   if (rc != SVO_OK) return rc;
+  populate_hits(hits, n);
   SVO_CUDA_TRY(cudaStreamSynchronize(st));
   return SVO_OK;
 }

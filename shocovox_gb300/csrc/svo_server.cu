@@ -14,9 +14,6 @@
 // work already running.
 #include <cuda_runtime.h>
 
-#include <sys/mman.h>
-#include <unistd.h>
-
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -110,18 +107,6 @@ __global__ void __launch_bounds__(256) copy_out_kernel(const __grid_constant__ C
     done = bytes / 4 * 4;
   }
   for (uint64_t k = done + at; k < bytes; k += step) dst[k] = src[k];
-}
-
-// Gives the pages under a result buffer memory, contents unchanged, before the device writes them: a page that
-// the device touches first costs it a fault (24 requests into fresh buffers: 23 ms against 8).  The
-// host does it while the cast runs.  Kernels without the call leave it to the device.
-void populate(void* p, uint64_t bytes) {
-#ifndef MADV_POPULATE_WRITE
-#define MADV_POPULATE_WRITE 23
-#endif
-  static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p) / page * page, b = reinterpret_cast<uintptr_t>(p) + bytes;
-  if (bytes) madvise(reinterpret_cast<void*>(a), (b - a + page - 1) / page * page, MADV_POPULATE_WRITE);
 }
 
 double now_s() {
