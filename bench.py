@@ -335,9 +335,16 @@ def interleaved_repeats(variants, steps, repeats, stream, torch):
     return out
 
 
-def batched_launches(items, sort_key):
+def cast_launches(items, sort_key):
     """Kernel launches of one svo_cast_batched call: the claim-order cast if any item is cast in claim
-    order, plus the ray sort's bin, three scan, scatter and cast launches if any item is sorted."""
+    order, and one for the unordered items (sort_key 1, no row length)."""
+    loose = [it for it in items if sort_key and not (len(it) > 4 and it[4]) and it[2]]
+    return (1 if any(it[2] and it not in loose for it in items) else 0) + (1 if loose else 0)
+
+
+def batched_launches(items, sort_key):
+    """The launches of the same call while sort_key 1 sorted the rays (bin, three scans, scatter, cast), which
+    records of that time count in."""
     sorted_items = [it for it in items if sort_key and not (len(it) > 4 and it[4]) and it[2]]
     claimed = [it for it in items if it[2] and it not in sorted_items]
     return (1 if claimed else 0) + (6 if sorted_items else 0)
@@ -345,7 +352,7 @@ def batched_launches(items, sort_key):
 
 def autotune_batched(svo, torch, ws, items, stream, fixed_sort=None):
     """The project's autotuner (shocovox_gb300.autotune, no cache) on `items`: threads per block x rays
-    per claim x ray-block shape (items with a row length) or ray-sort key (items without), then the
+    per claim x ray-block shape (items with a row length) or sort key (items without), then the
     staging depth of the best.  fixed_sort: only configurations with that sort key are kept.
     Returns (LaunchConfig, {config string: ms})."""
     from shocovox_gb300 import autotune
@@ -505,7 +512,7 @@ def run_single(args, w, workload):
         bms = interleaved_repeats({"b": lambda: ws.cast(items, cfg, s)}, args.steps, 1, stream, torch)["b"][0]
         variants = {"persistent_autotuned": dict({"value": round(n / (bms / 1e3) / 1e6, 3), "unit": "Mrays/s",
                                                   "ms_per_step": round(bms, 4),
-                                                  "launches_per_step": batched_launches(items, cfg.sort_key)},
+                                                  "launches_per_step": cast_launches(items, cfg.sort_key)},
                                                  **cfg_record(cfg)),
                     "sweep_ms": sweep,
                     "plain_staging_depth_sweep": stage_sweep,
@@ -623,7 +630,7 @@ def run_single(args, w, workload):
 # ---- comparison (a): incoherent rays, plain cast vs batched forms ---------------------------------
 def compare_incoherent(args):
     """incoherent1024: plain svo_cast against the autotuned persistent batched cast in index order and
-    with the ray sort, timed over interleaved repeats, every variant's hits checked against the oracle."""
+    with sort key 1, timed over interleaved repeats, every variant's hits checked against the oracle."""
     import torch
     import shocovox_gb300 as svo
     w = WORKLOADS["incoherent1024"]
@@ -682,7 +689,7 @@ def compare_incoherent(args):
                                    sweep_ms={"park_below%d" % t: round(v[0], 4) for t, v in t_sweep.items()})}
     for v in ("index_order", "sorted"):
         c = best[v]
-        res["batched_" + v] = dict(spread(n, reps[v]), launches_per_step=batched_launches(items[v], c.sort_key),
+        res["batched_" + v] = dict(spread(n, reps[v]), launches_per_step=cast_launches(items[v], c.sort_key),
                                    vs_plain=versus(spread(n, reps[v]), plain), autotune_sweep_ms=sweeps[v],
                                    **cfg_record(c))
     del outs, rays
@@ -937,9 +944,9 @@ def run_multiscene(args, w):
                    "voxels_inserted": n_voxels, "gen_s": round(gen_s, 1), "build_s": round(build_s, 1),
                    "l2": "rays %.0f MB + hits %.0f MB per step (larger than L2)" % (total * 24 / 1e6, total * 34 / 1e6),
                    "timed": "the batched cast replayed from a CUDA graph (one persistent launch; with sort_key 1 the "
-                            "ray sort's six launches too), median of %d repeats of %d steps" % (REPEATS, args.steps),
+                            "unordered items' launch too), median of %d repeats of %d steps" % (REPEATS, args.steps),
                    "ray_order": "per scene: camera rays as rows of the image (8 x 4 ray blocks per warp), "
-                                "random rays in order or sorted by direction octant and entry point (autotune.sort_key)",
+                                "random rays in index order or a step of each at a time (autotune.sort_key)",
                    "graph": graph_sp,
                    "serial_plain": dict(serial_sp, launches_per_step=len(items)),
                    "batched": batched_sp,
@@ -952,7 +959,7 @@ def run_multiscene(args, w):
         "e2e": {"value": round(total / e2e_s / 1e6, 3), "unit": "Mrays/s", "h2d_bytes_per_step": total * 24,
                 "d2h_bytes_per_step": total * sum(OUT_BYTES.values()),
                 "how": "4 groups of items, each copy-in, batched launch, copy-out on its own stream"},
-        "gpu_launches": args.steps * batched_launches(items, gcfg.sort_key),
+        "gpu_launches": args.steps * cast_launches(items, gcfg.sort_key),
         "clocks": clk,
         "parity": parity,
     }

@@ -3,10 +3,9 @@
 Sweeps threads per block, rays per warp grab, persistent CTAs per SM, for
 batches with camera images (items with a row length) the shape of the ray
 blocks a warp casts together, and for batches with rays in no particular order
-(items without a row length) the ray-sort key, on the caller's own batch; then,
+(items without a row length) the sort key, on the caller's own batch; then,
 for the fastest of those, the staging depth (top tree levels every block copies
-into shared memory) and, when it sorts, the lane-refill threshold of the sorted
-cast.  Keeps the fastest and caches the choice per (GPU name,
+into shared memory) and, with sort key 1, the lane-refill threshold.  Keeps the fastest and caches the choice per (GPU name,
 workload signature) in a JSON file next to the built library, so later runs skip
 the sweep.
 """
@@ -21,9 +20,9 @@ BLOCKS = (64, 96, 128)
 CHUNKS = (32, 64, 128)
 PER_SM = (0,)  # 0 = as many as occupancy allows
 SHAPES = (3, 4)  # ray blocks of 8 x 4 or 16 x 2 for items with a row length
-SORT_KEYS = (0, 1)  # index order, or sorted by direction octant and entry point
+SORT_KEYS = (0, 1)  # 32 neighbours at a time, or a step of each ray at a time
 STAGING = (1, 2, 3, 4)  # staging depths tried on the best configuration found at depth 0
-REFILL = (16, 24, 32)  # lane-refill thresholds tried on the best sorted configuration
+REFILL = (16, 24, 32)  # lane-refill thresholds tried on the best configuration with sort key 1
 
 
 def _load():
@@ -71,7 +70,7 @@ def tune(ws, items, gpu_name, time_fn, use_cache=True):
     for st in STAGING:
         table["%dx%dx%dx%dx%dx%dx0" % (b, c, p, sh, so, st)] = time_fn(_lib.LaunchConfig(b, c, p, sh, so, st, 0))
     if so == 1:
-        # the sorted cast: its lane-refill threshold at the best staging depth, for every block size (each
+        # sort key 1: its lane-refill threshold at the best staging depth, for every block size (each
         # with its best rays per claim): the refilling kernel's occupancy is not the plain kernel's, so the
         # best block without refill need not be the best with it
         st = int(min((k for k in table if k.startswith("%dx%dx%dx%dx%dx" % (b, c, p, sh, so))), key=table.get).split("x")[5])
