@@ -71,3 +71,7 @@ extern "C" void flow_check(svo_scene* sc, const float* o, const float* d, uint64
     std::memcpy(rec + 5, fl, sizeof(fl));
   }
 }
+
+// The rays that tell a batch's order (rays_mixed): the first of pair k of n rays.
+extern "C" uint64_t flow_pair(uint64_t n, uint32_t k) { return pair_at(n, k); }
+extern "C" uint32_t flow_pair_apart() { return kPairApart; }

@@ -113,3 +113,21 @@ def test_rays_left_to_the_general_forms(flow, oracle_mod):
     flow.flow_check(h, vp(o), vp(d), ctypes.c_uint64(len(o)), vp(form), vp(rec))
     assert [int(v != 0) for v in form] == [c[2] for c in cases]
     flow.svo_scene_destroy(h)
+
+
+@pytest.mark.parametrize("width", [96, 127, 240, 320, 640, 960, 1024, 1280, 1283, 1920, 2048, 2560, 3840, 4096])
+def test_sampled_pairs_of_an_image_stay_in_their_rows(flow, width):
+    """At most 8 of the 32 pairs may straddle a row's end, or a camera's rays would be cast as rays in no order."""
+    flow.flow_pair.restype, flow.flow_pair.argtypes = ctypes.c_uint64, [ctypes.c_uint64, ctypes.c_uint32]
+    apart = flow.flow_pair_apart()
+    for ratio in (9 / 16, 3 / 4, 1):
+        rows = int(width * ratio)
+        for images in range(1, 33):
+            n = width * rows * images
+            if n < 1 << 19:
+                continue
+            at = [flow.flow_pair(n, k) for k in range(32)]
+            assert all(a < b for a, b in zip(at, at[1:])) and at[-1] + apart < n
+            assert sum(a % width + apart >= width for a in at) <= 8, (width, rows, images)
+    for n in (1, 8, 9, 31, 40, 41, 64, 1 << 19, 1 << 33):
+        assert all(flow.flow_pair(n, k) + (apart if n > apart else 0) < n for k in range(32)), n
