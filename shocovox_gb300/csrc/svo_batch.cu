@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128, 6)
   __shared__ FlowShared sh;
   __shared__ FlowLists<BatchRayId> lists[4];
   FlowLists<BatchRayId>& w = lists[threadIdx.x >> 5];
-  unsigned long long c = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
+  unsigned long long c = flow_claim(queue);
   while (uint32_t others = flow_cast(src, claims, refill, queue, c, sh, w)) {
     for (uint32_t k = threadIdx.x & 31u; k < others; k += 32u) {
       const BatchRayId id = w.other[k];

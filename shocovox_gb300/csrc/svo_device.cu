@@ -214,6 +214,17 @@ struct FlowBlock {
   FlowShared sh;
   FlowLists<RayId> lists[4];
 };
+// The block's answer.  Hits may be written over the rays, and a block that starts late reads some of them: blocks may
+// answer differently, the warps of one may not (their lists share memory).
+__device__ __forceinline__ bool block_mixed(const ArraySource& src) {
+  __shared__ uint32_t mixed;
+  if (threadIdx.x < 32u) {
+    const bool x = rays_mixed(src.rays, src.n, src.s);
+    if (threadIdx.x == 0u) mixed = x;
+  }
+  __syncthreads();
+  return mixed != 0u;
+}
 // 6 blocks per SM (80 registers): at 7 both casts' loops spill, and a camera's 925 K rays on 256^3 take 256 us
 // instead of 241 (243 in queue_kernel's own launch), 2^22 random rays on 512^3 642 us instead of 679.
 __global__ void __launch_bounds__(128, 6)
@@ -224,13 +235,13 @@ __global__ void __launch_bounds__(128, 6)
     WaitingRays waiting[4];
     __device__ U() {}
   } m;
-  if (test && !rays_mixed(src.rays, src.n, src.s)) {
+  if (test && !block_mixed(src)) {
     queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
     return;
   }
   const uint32_t lane = threadIdx.x & 31u;
   FlowLists<RayId>& lists = m.flow.lists[threadIdx.x >> 5];
-  unsigned long long c = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
+  unsigned long long c = flow_claim(queue);
   while (uint32_t others = flow_cast(src, src.order.claims, refill, queue, c, m.flow.sh, lists)) {
     for (uint32_t k = lane; k < others; k += 32u) {
       const RayId id = lists.other[k];

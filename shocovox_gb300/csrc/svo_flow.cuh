@@ -333,7 +333,8 @@ struct FlowLists {
 //   ray(id, o, d)              its origin and direction
 //   scene(id)                  its scene
 //   put(id, h)                 writes its record
-// c is the warp's next claim (the first is its own number, further ones come from the counter queue[0]).
+// c is the warp's next claim, from the counter queue[0] like queue_cast's: whichever of the two a block runs, each
+// claim is cast once.
 // Returns how many rays wait in w.other for the general forms: 0 once the batch is done.  Where there are
 // some the caller casts them and calls again (no ray is in flight then, so their registers are free).
 //
@@ -345,12 +346,17 @@ struct FlowLists {
 // step code -- so rays that have nothing in common still run most instructions together.
 constexpr uint32_t kFlowRefill = 12;  // 8 to 16 measured alike
 
+__device__ __forceinline__ unsigned long long flow_claim(unsigned long long* __restrict__ queue) {
+  unsigned long long c = 0;
+  if ((threadIdx.x & 31u) == 0u) c = atomicAdd(queue, 1ull);
+  return __shfl_sync(0xFFFFFFFFu, c, 0);
+}
+
 template <class Src, class Id>
 __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, uint32_t refill,
                                               unsigned long long* __restrict__ queue, unsigned long long& c,
                                               FlowShared& sh, FlowLists<Id>& w) {
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  const uint64_t warps = (uint64_t)gridDim.x * 4u;
   uint32_t tid = threadIdx.x;
   asm volatile("" : "+r"(tid));  // kept in a register: each use read the special register again (680 -> 665 us)
   uint32_t count = 0, others = 0;  // rays in the lists (the same in every lane)
@@ -412,8 +418,7 @@ __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, u
       if (other) w.other[__popc(mo & below)] = id;
       count += __popc(mu);
       others = __popc(mo);
-      if (lane == 0) c = atomicAdd(queue, 1ull) + warps;
-      c = __shfl_sync(0xFFFFFFFFu, c, 0);
+      c = flow_claim(queue);
     }
     __syncwarp();
     const uint32_t take = count < need ? count : need;

@@ -63,6 +63,31 @@ def test_sizes_around_the_lines(oracle_mod, n):
         assert_same_hits(device_cast(p, origins, dirs), ref, label="%s %d" % (label, n))
 
 
+@pytest.mark.parametrize("order", ["random", "camera"])
+def test_points_written_over_the_origins(oracle_mod, order):
+    """A block that starts late tells the rays' order from some that are hit points already: each ray is cast once all the same."""
+    torch = pytest.importorskip("torch")
+    o, p = both(oracle_mod, 64, 4, svo.gen_scene(0, 64, 4, seed=5, spheres=3, octaves=2, base_freq=1 / 16, height_lo=2.0,
+                                                 height_hi=24.0))
+    n = 3 * FLOW
+    if order == "random":
+        origins, dirs = random_rays(np.random.default_rng(4), 64, n)
+    else:
+        origins, dirs = (a[:n] for a in svo.gen_camera_rays([150.0, 90.0, 140.0], [32.0, 16.0, 32.0], 50.0, 1536, 1024))
+    ref = o.cast(origins, dirs, threads=16)
+    cols = {k: torch.from_numpy(np.ascontiguousarray(a[:, i])).cuda()
+            for a, names in ((origins, ("ox", "oy", "oz")), (dirs, ("dx", "dy", "dz"))) for i, k in enumerate(names)}
+    status = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    p.cast({k: v.data_ptr() for k, v in cols.items()},
+           {"status": status.data_ptr(), **{"p" + a: cols["o" + a].data_ptr() for a in "xyz"}}, n,
+           torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert np.array_equal(status.cpu().numpy(), ref["status"])
+    hit = ref["status"] == 1
+    for a in "xyz":
+        assert np.array_equal(cols["o" + a].cpu().numpy()[hit].view(np.uint32), ref["p" + a][hit].view(np.uint32)), a
+
+
 def test_heads_follow_in_place_syncs(oracle_mod):
     rng = np.random.default_rng(9)
     o, p = both(oracle_mod, 64, 4, svo.gen_scene(3, 64, 4, seed=6, occupancy=0.05, spheres=2))
