@@ -104,10 +104,9 @@ struct WaitingRays {  // the ray's origin and direction are read again from the 
 template <bool kCount, bool kLod = false, bool kStage = false>
 __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& rays, const HitsView& out, uint64_t n,
                                            const ClaimOrder& order, unsigned long long* __restrict__ queue,
-                                           const SharedLuts& L, WaitingRays (&waiting)[4], const DevNode* stg,
+                                           const SharedLuts& L, WaitingRays& w, const DevNode* stg,
                                            float viewing_distance = 0.0f, uint32_t stage_n = 0, uint32_t pack = 32u) {
   const uint32_t lane = threadIdx.x & 31u;
-  WaitingRays& w = waiting[threadIdx.x >> 5];
   uint32_t count = 0;  // rays waiting (the same in every lane)
   bool more = true;    // claims left
   for (;;) {
@@ -202,47 +201,37 @@ __global__ void __launch_bounds__(128, 7)
     fill_shared_luts(L);
     stage_records(stg, s.top, stage_n);
     __syncthreads();
-    queue_cast<kCount, kLod, kStage>(s, rays, out, n, order, queue, L, waiting, stg, viewing_distance, stage_n, pack);
+    queue_cast<kCount, kLod, kStage>(s, rays, out, n, order, queue, L, waiting[threadIdx.x >> 5], stg, viewing_distance, stage_n, pack);
   } else {
-    queue_cast<kCount, kLod>(s, rays, out, n, order, queue, kLuts, waiting, nullptr, viewing_distance, 0, pack);
+    queue_cast<kCount, kLod>(s, rays, out, n, order, queue, kLuts, waiting[threadIdx.x >> 5], nullptr, viewing_distance, 0, pack);
   }
 }
 
 // A large batch without a row layout: a camera's rays in raster order, which queue_cast casts, or rays in
 // no order, which flow_cast casts but for those of the general forms.  The rays themselves tell (rays_mixed).
-struct FlowBlock {
-  FlowShared sh;
-  FlowLists<RayId> lists[4];
+// Hits may be written over the rays, and a warp that starts late reads some of them: warps may answer differently.  So they
+// share no memory, and both casts take their claims from one counter.
+union PlainLists {  // one warp's
+  FlowLists<RayId> flow;
+  WaitingRays waiting;
+  __device__ PlainLists() {}
 };
-// The block's answer.  Hits may be written over the rays, and a block that starts late reads some of them: blocks may
-// answer differently, the warps of one may not (their lists share memory).
-__device__ __forceinline__ bool block_mixed(const ArraySource& src) {
-  __shared__ uint32_t mixed;
-  if (threadIdx.x < 32u) {
-    const bool x = rays_mixed(src.rays, src.n, src.s);
-    if (threadIdx.x == 0u) mixed = x;
-  }
-  __syncthreads();
-  return mixed != 0u;
-}
 // 6 blocks per SM (80 registers): at 7 both casts' loops spill, and a camera's 925 K rays on 256^3 take 256 us
 // instead of 241 (243 in queue_kernel's own launch), 2^22 random rays on 512^3 642 us instead of 679.
 __global__ void __launch_bounds__(128, 6)
     plain_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ queue, uint32_t refill,
                  bool test) {
-  __shared__ union U {
-    FlowBlock flow;
-    WaitingRays waiting[4];
-    __device__ U() {}
-  } m;
-  if (test && !block_mixed(src)) {
+  __shared__ FlowShared sh;
+  __shared__ PlainLists lists_of[4];
+  PlainLists& m = lists_of[threadIdx.x >> 5];
+  if (test && !rays_mixed(src.rays, src.n, src.s)) {
     queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
     return;
   }
   const uint32_t lane = threadIdx.x & 31u;
-  FlowLists<RayId>& lists = m.flow.lists[threadIdx.x >> 5];
+  FlowLists<RayId>& lists = m.flow;
   unsigned long long c = flow_claim(queue);
-  while (uint32_t others = flow_cast(src, src.order.claims, refill, queue, c, m.flow.sh, lists)) {
+  while (uint32_t others = flow_cast(src, src.order.claims, refill, queue, c, sh, lists)) {
     for (uint32_t k = lane; k < others; k += 32u) {
       const RayId id = lists.other[k];
       float o[3], d[3];

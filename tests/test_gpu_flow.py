@@ -65,7 +65,7 @@ def test_sizes_around_the_lines(oracle_mod, n):
 
 @pytest.mark.parametrize("order", ["random", "camera"])
 def test_points_written_over_the_origins(oracle_mod, order):
-    """A block that starts late tells the rays' order from some that are hit points already: each ray is cast once all the same."""
+    """A warp that starts late tells the rays' order from some that are hit points already: each ray is cast once all the same."""
     torch = pytest.importorskip("torch")
     o, p = both(oracle_mod, 64, 4, svo.gen_scene(0, 64, 4, seed=5, spheres=3, octaves=2, base_freq=1 / 16, height_lo=2.0,
                                                  height_hi=24.0))
