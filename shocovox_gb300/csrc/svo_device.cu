@@ -16,6 +16,7 @@
 #include "svo_cast.cuh"
 #include "svo_flow.cuh"
 #include "svo_queue.h"
+#include "svo_route.h"
 #include "svo_trace.h"
 
 namespace svo {
@@ -1278,9 +1279,13 @@ svo_status svo_cast_host_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, u
     int dev = 0;
     SVO_CUDA_TRY(cudaGetDevice(&dev));
     SVO_CUDA_TRY(cudaDeviceGetAttribute(&direct, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev));
+    const bool aligned = arrays_aligned(*rays, *hits);
     if (g_host_transfer == 2 && !direct)
       return fail(SVO_ERR_ARGUMENT, "svo_cast_host: this device cannot access host memory directly");
+    if (g_host_transfer == 2 && !aligned)
+      return fail(SVO_ERR_ARGUMENT, "svo_cast_host: the device cannot access arrays off their element's alignment directly");
     if (g_host_transfer == 0 && row_length < 16 && n >= kQueueMinRays) direct = 0;
+    if (!aligned) direct = 0;
   }
   if (!direct) return cast_host_pipelined(sc, rays, n, hits, st, row_length);
   const svo_status rc = launch_cast(sc, rays, n, hits, st, row_length, true);
