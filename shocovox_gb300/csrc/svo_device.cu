@@ -1285,7 +1285,7 @@ svo_status svo_cast_host_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, u
     if (g_host_transfer == 2 && !aligned)
       return fail(SVO_ERR_ARGUMENT, "svo_cast_host: the device cannot access arrays off their element's alignment directly");
     if (g_host_transfer == 0 && row_length < 16 && n >= kQueueMinRays) direct = 0;
-    if (!aligned) direct = 0;
+    if (!aligned || (g_host_transfer == 0 && hits_over_rays(*rays, *hits, n))) direct = 0;
   }
   if (!direct) return cast_host_pipelined(sc, rays, n, hits, st, row_length);
   const svo_status rc = launch_cast(sc, rays, n, hits, st, row_length, true);

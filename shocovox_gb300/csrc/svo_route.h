@@ -19,4 +19,21 @@ inline bool arrays_aligned(const svo_rays& rays, const svo_hits& hits) {
   return true;
 }
 
+// Whether hits written in place may change rays that are still to be read: a hit field over a ray array, other than element
+// for element (a ray is read before its own hit is written).  Copies of a batch are complete before its cast.
+inline bool hits_over_rays(const svo_rays& rays, const svo_hits& hits, uint64_t n) {
+  const float* const in[6] = {rays.ox, rays.oy, rays.oz, rays.dx, rays.dy, rays.dz};
+  void* const* out = reinterpret_cast<void* const*>(&hits);
+  for (int f = 0; f < kHitFields; ++f) {
+    const uintptr_t h = reinterpret_cast<uintptr_t>(out[f]);
+    if (!h) continue;
+    for (const float* p : in) {
+      const uintptr_t r = reinterpret_cast<uintptr_t>(p);
+      if (h == r && kHitFieldBytes[f] == sizeof(float)) continue;
+      if (h < r + sizeof(float) * n && r < h + kHitFieldBytes[f] * n) return true;
+    }
+  }
+  return false;
+}
+
 }  // namespace svo

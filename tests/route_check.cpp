@@ -5,4 +5,6 @@ extern "C" {
 
 int route_aligned(const svo_rays* rays, const svo_hits* hits) { return svo::arrays_aligned(*rays, *hits) ? 1 : 0; }
 
+int route_overlap(const svo_rays* rays, const svo_hits* hits, uint64_t n) { return svo::hits_over_rays(*rays, *hits, n) ? 1 : 0; }
+
 }  // extern "C"

@@ -54,3 +54,24 @@ def test_in_place_access_of_unaligned_arrays_is_refused(scene):
             p.cast_host_soa(cols, out)
     finally:
         svo.check(svo.lib().svo_set_host_transfer(0))
+
+
+@pytest.mark.parametrize("n", [2, 1000, 20000])
+@pytest.mark.parametrize("field,off", [("status", 0), ("brick_octant", 1), ("px", 0), ("px", 4), ("albedo", -4), ("nz", 400),
+                                       ("entry_kind", -1)])
+def test_hits_over_the_rays(scene, n, field, off):
+    """A field that lies over a ray array, element for element or not."""
+    o, p = scene
+    origins, dirs = random_rays(np.random.default_rng(n), 64, n)
+    ref = o.cast(origins, dirs, threads=16)
+    raw = np.zeros(6 * 4 * n + 4096, np.uint8)  # the six ray arrays, one after the other
+    base = (-raw.ctypes.data) % 16 + 1024
+    cols = [raw[base + 4 * n * k:base + 4 * n * (k + 1)].view(np.float32) for k in range(6)]
+    for k, c in enumerate(cols):
+        c[...] = origins[:, k] if k < 3 else dirs[:, k - 3]
+    at = base + 4 * n * 1 + off  # over oy
+    out = {k: np.zeros(n, t) for k, t in svo.HIT_FIELDS.items() if k != field}
+    kind = np.dtype(svo.HIT_FIELDS[field])
+    out[field] = raw[at:at + kind.itemsize * n].view(kind)
+    p.cast_host_soa(cols, out)
+    assert_same_hits(out, ref, counters=True, label="%s at %d" % (field, off))

@@ -47,3 +47,22 @@ def test_alignment_of_host_arrays(route):
     for k, t in svo.HIT_FIELDS.items():
         for off in (1, 2, 3):
             assert aligned(**{k: 0x900000 + off}) == (np.dtype(t).itemsize == 1), (k, off)
+
+
+def test_overlap_of_host_arrays(route):
+    n = 100
+
+    def over(n=n, **change):
+        r, h = arrays(**change)
+        return route.route_overlap(ctypes.byref(r), ctypes.byref(h), ctypes.c_uint64(n)) == 1
+
+    assert not over() and not over(**{k: 0 for k in svo.HIT_FIELDS})
+    at = 0x10000 + 0x10000 * 2  # oz
+    for k, t in svo.HIT_FIELDS.items():
+        size = np.dtype(t).itemsize
+        assert over(**{k: at}) == (size == 1), k  # element for element, or not
+        for off in (-size * n + 1, -4, -1, 1, 4, 4 * n - 1):
+            assert over(**{k: at + off}) == (-size * n < off), (k, off)
+        for off in (-size * n, 4 * n):
+            assert not over(**{k: at + off}), (k, off)
+        assert not over(0, **{k: at + 4})
