@@ -215,8 +215,9 @@ svo_status svo_set_device_allocator(svo_alloc_fn alloc, svo_free_fn release, voi
  * counter that the scene keeps per stream (up to 64 streams; casts on further streams, and on
  * cudaStreamPerThread, use one thread per ray).  From 524,288 rays on, rays without a row layout that
  * go their own ways (a sample of them is looked at on the device) are cast a step of each at a time.  Casts of one scene on different streams may
- * overlap.  A CUDA graph that captured a cast reuses the counter of the stream it was captured
- * on: do not run it concurrently with casts on that stream. */
+ * overlap.  A CUDA graph that captured a cast uses a counter of the stream it was captured on: do not run it
+ * concurrently with itself, or with another graph captured on that stream (the hits of those two casts would be
+ * incomplete, later ones' not). */
 svo_status svo_cast(svo_scene* scene, const svo_rays* rays, uint64_t n, const svo_hits* hits, void* stream);
 /* Octree::get_by_ray_at_lod (raytracing_on_cpu.rs:325-565): with MIP maps enabled (svo_mip_switch) a
  * node's MIP brick is read once its level is below (origin - p rounded to the level's grid).length()

@@ -21,6 +21,7 @@
 
 #include "svo_cast.cuh"
 #include "svo_flow.cuh"
+#include "svo_queue.h"
 #include "svo_trace.h"
 
 namespace svo {
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(128, 6)
   __shared__ FlowShared sh;
   __shared__ FlowLists<BatchRayId> lists[4];
   FlowLists<BatchRayId>& w = lists[threadIdx.x >> 5];
+  queue_begin(queue);
   unsigned long long c = flow_claim(queue);
   while (uint32_t others = flow_cast(src, claims, refill, queue, c, sh, w)) {
     for (uint32_t k = threadIdx.x & 31u; k < others; k += 32u) {
@@ -307,7 +309,6 @@ __global__ void __launch_bounds__(128, 6)
     }
     __syncwarp();
   }
-  queue_done(queue, (uint64_t)gridDim.x * 4u);
 }
 
 }  // namespace svo
@@ -348,7 +349,8 @@ svo_status launch_claimed(const BatchItemDev* d_items, uint32_t n_items, uint64_
 // pinned host staging copy of the table.  Grows only when the item count grows.
 struct svo_batch_workspace {
   svo::BatchItemDev* d_items = nullptr;
-  unsigned long long* d_counter = nullptr;  // [0] claim-order work counter, [2] and [3] batch_flow_kernel's queue
+  unsigned long long* d_counter = nullptr;  // [0] claim-order work counter, from [2] on the words of the loose items' launches
+  svo::QueueTurn turn;
   svo::BatchItemDev* h_items = nullptr;     // pinned
   svo::LooseItemDev* d_loose = nullptr;     // the items of batch_flow_kernel
   svo::LooseItemDev* h_loose = nullptr;     // pinned
@@ -367,8 +369,8 @@ svo_status svo_batch_workspace_create(svo_batch_workspace** out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ws->sm_count, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaMalloc(&ws->d_counter, 4 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(ws->d_counter, 0, 4 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&ws->d_counter, (2 + kQueueWords) * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMemset(ws->d_counter, 0, (2 + kQueueWords) * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // casts may follow on any stream
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->copied, cudaEventDisableTiming);
   if (e != cudaSuccess) {
@@ -475,11 +477,12 @@ svo_status svo_cast_batched(svo_batch_workspace* ws, const svo_batch_item* items
   if (!in_capture) SVO_CUDA_TRY(cudaEventRecord(ws->copied, st));
   if (n_loose) {
     const uint32_t below = refill ? 33u - refill : kFlowRefill;
-    unsigned long long* queue = ws->d_counter + 2;
+    QueueLaunch take;
+    SVO_CUDA_TRY(queue_take({ws->d_counter + 2, &ws->turn}, st, take));
     const uint32_t per_sm = cfg ? cfg->blocks_per_sm : 0;
     if (n_loose == 1) {
       const BatchItemDev& d = ws->h_items[one];
-      const svo_status rc = launch_plain(d.scene, d.rays, d.hits, items[one].n, below, per_sm, queue, st);
+      const svo_status rc = launch_plain(d.scene, d.rays, d.hits, items[one].n, below, per_sm, take.word, st);
       if (rc != SVO_OK) return rc;
     } else {
       int per = (int)per_sm;
@@ -489,9 +492,10 @@ svo_status svo_cast_batched(svo_batch_workspace* ws, const svo_batch_item* items
       }
       const uint64_t grid = std::min<uint64_t>((uint64_t)ws->sm_count * (uint64_t)per, (loose_claims + 3) / 4);
       batch_flow_kernel<<<(unsigned)grid, 128, 0, st>>>(BatchSource{ws->d_items, ws->d_loose, n_items}, loose_claims, below,
-                                                        queue);
+                                                        take.word);
       SVO_CUDA_TRY(cudaGetLastError());
     }
+    take.launched();
   }
   if (total == 0) return SVO_OK;
   return launch_claimed(ws->d_items, n_items, total, ws->d_counter, chunk, block, cfg, count, staged_n, ws->sm_count, st);

@@ -82,15 +82,6 @@ inline uint32_t pack_target(uint64_t claims, uint64_t warps) {
   return (uint32_t)std::min<uint64_t>(32u, std::max<uint64_t>(4u, 5u * claims / std::max<uint64_t>(warps, 1u)));
 }
 
-// A warp has taken its last claim: the last of the launch's `warps` warps zeroes the claim counter
-// queue[0] and the count of finished warps queue[1] for the next launch on the stream.
-__device__ __forceinline__ void queue_done(unsigned long long* queue, uint64_t warps) {
-  if ((threadIdx.x & 31u) == 0u && atomicAdd(queue + 1, 1ull) == warps - 1u) {
-    queue[0] = 0;
-    queue[1] = 0;
-  }
-}
-
 // ------------------------------------------------------------------ Rust f32 semantics
 __device__ __forceinline__ float rmin(float a, float b) { return isnan(a) ? b : (isnan(b) ? a : (b < a ? b : a)); }
 __device__ __forceinline__ float rmax(float a, float b) { return isnan(a) ? b : (isnan(b) ? a : (b > a ? b : a)); }

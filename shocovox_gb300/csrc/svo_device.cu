@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(128, 7)
 // Queued cast: a persistent grid whose warps claim 32 rays at a time from a work counter.  The
 // cost of a ray varies by orders of magnitude (a sky ray leaves after a few node visits, a
 // grazing ray walks a whole cave), and a warp that finishes early takes more work instead of
-// idling until its block's slowest warp is done.  The counter (claims taken) starts at 0, and the last
-// warp to finish zeroes it for the next launch (queue_done).
+// idling until its block's slowest warp is done.  The counter (claims taken) starts at 0, and the kernel
+// zeroes the one of the next launch (queue_begin).
 //
 // Rays that miss the octree's root box get their miss written at once.  A claim whose rays all
 // enter is cast as it is; the entering rays of other claims wait in the warp's slice of shared
@@ -187,7 +187,6 @@ __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& r
     write_hit(s, out, i, h);
     if (kCount) write_counters(out, i, h);
   }
-  queue_done(queue, (uint64_t)gridDim.x * 4u);
 }
 
 template <bool kCount, bool kLod = false, bool kStage = false>
@@ -195,6 +194,7 @@ __global__ void __launch_bounds__(128, 7)
     queue_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
                  unsigned long long* __restrict__ queue, float viewing_distance, uint32_t stage_n, uint32_t pack) {
   __shared__ WaitingRays waiting[4];
+  queue_begin(queue);
   if constexpr (kStage) {
     __shared__ SharedLuts L;
     extern __shared__ uint4 staged_smem[];
@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(128, 6)
   __shared__ FlowShared sh;
   __shared__ PlainLists lists_of[4];
   PlainLists& m = lists_of[threadIdx.x >> 5];
+  queue_begin(queue);
   if (test && !rays_mixed(src.rays, src.n, src.s)) {
     queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
     return;
@@ -244,7 +245,6 @@ __global__ void __launch_bounds__(128, 6)
     }
     __syncwarp();
   }
-  queue_done(queue, (uint64_t)gridDim.x * 4u);
 }
 
 // Host-buffer cast that reads its rays from and writes its hits to host memory in place (over the CPU
@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(128, 7)
   __shared__ PairStage stage[4];
   const uint32_t lane = threadIdx.x & 31u;
   PairStage& ps = stage[threadIdx.x >> 5];
+  queue_begin(queue);
   const uint64_t warps = (uint64_t)gridDim.x * 4u;
   for (unsigned long long c = ((uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5)) * 2u; c < order.claims;) {
     for (uint32_t half = 0; half < 2; ++half) {
@@ -333,7 +334,6 @@ __global__ void __launch_bounds__(128, 7)
     if (lane == 0) c = atomicAdd(queue, 2ull) + 2u * warps;
     c = __shfl_sync(0xFFFFFFFFu, c, 0);
   }
-  queue_done(queue, warps);
 }
 
 // Below this many rays one grid with fewer rays per warp (grid_lanes) is faster than the work queue: 119,860 camera
@@ -354,6 +354,7 @@ void destroy_queues(DeviceImage& d) {
 svo_status create_queues(DeviceImage& d, cudaStream_t st) {
   if (d.queues) return SVO_OK;
   CastQueues* q = new CastQueues();
+  const size_t bytes = (size_t)kQueueSlots * kQueueWords * sizeof(unsigned long long);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&q->sm_count, cudaDevAttrMultiProcessorCount, dev);
@@ -361,8 +362,8 @@ svo_status create_queues(DeviceImage& d, cudaStream_t st) {
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_count, queue_kernel<true>, 128, 0);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_plain, plain_kernel, 128, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&q->counters, 2 * kQueueSlots * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemsetAsync(q->counters, 0, 2 * kQueueSlots * sizeof(unsigned long long), st);
+  if (e == cudaSuccess) e = cudaMalloc(&q->counters, bytes);
+  if (e == cudaSuccess) e = cudaMemsetAsync(q->counters, 0, bytes, st);
   if (e != cudaSuccess) {
     cudaFree(q->counters);
     delete q;
@@ -902,7 +903,7 @@ uint32_t grid_lanes(uint64_t n) {
 }
 
 }  // namespace
-// plain_kernel over one batch whose rays are in no order (svo_batch.cu).  `queue`: two device words, zero.
+// plain_kernel over one batch whose rays are in no order (svo_batch.cu).  `queue`: its claim word (svo_queue.h).
 svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView& hits, uint64_t n, uint32_t refill,
                         uint32_t blocks_per_sm, unsigned long long* queue, cudaStream_t st) {
   int dev = 0, sms = 0, per = (int)blocks_per_sm;
@@ -931,7 +932,10 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
   CastQueues* q = sc->dev.queues;
   if (q && n >= kQueueMinRays) {
     std::lock_guard<std::mutex> lock(q->m);
-    if (unsigned long long* queue = queue_counter(q, st)) {
+    if (const QueueWords words = queue_words(q, st); words.words) {
+      QueueLaunch take;
+      SVO_CUDA_TRY(queue_take(words, st, take));
+      unsigned long long* const queue = take.word;
       const int per_sm = std::max(1, count ? q->blocks_per_sm_count : q->blocks_per_sm);
       const uint64_t resident = (uint64_t)q->sm_count * per_sm;
       const ClaimOrder order = claim_order(n, row, in_place ? 4 : 3);
@@ -966,6 +970,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, true);
       }
       SVO_CUDA_TRY(cudaGetLastError());
+      take.launched();
       return SVO_OK;
     }
   }
@@ -1226,8 +1231,8 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
   const HitsView hv = hits_view_of(*hits);
   const bool count = counts_requested(*hits);
   std::lock_guard<std::mutex> lock(q->m);
-  unsigned long long* queue = queue_counter(q, st);
-  if (!queue) {
+  const QueueWords words = queue_words(q, st);
+  if (!words.words) {
     const uint64_t blocks = (n + 127) / 128;
     if (blocks > 0x7FFFFFFFull) return fail(SVO_ERR_ARGUMENT, "svo_cast_lod: too many rays for one launch");
     if (count)
@@ -1244,11 +1249,14 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
   const ClaimOrder order = claim_order(n, row);
   const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * per_sm, (order.claims + 3) / 4);
   const uint32_t pack = pack_target(order.claims, (uint64_t)q->sm_count * per_sm * 4u);
+  QueueLaunch take;
+  SVO_CUDA_TRY(queue_take(words, st, take));
   if (count)
-    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance, 0, pack);
+    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack);
   else
-    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, queue, viewing_distance, 0, pack);
+    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack);
   SVO_CUDA_TRY(cudaGetLastError());
+  take.launched();
   return SVO_OK;
 }
 

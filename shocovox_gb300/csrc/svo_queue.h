@@ -1,10 +1,12 @@
 // svo_queue.h -- the per-stream work counters of a scene, shared by the queued cast
 // (svo_device.cu) and the fused render (svo_render.cu).
 //
-// A queued kernel's warps claim work from a counter that starts at 0 and that the launch's last warp
-// zeroes again (queue_done, svo_cast.cuh), so a launch needs nothing before it.  Launches on one
-// stream run one after another, so a stream can reuse its counter; launches on different streams
-// may overlap, so every stream that uses the scene gets a counter of its own.
+// A queued kernel's warps claim work from a counter word that starts at 0.  Launches on one stream run one after
+// another, so a stream takes two words in turn, and a launch zeroes the next one's (queue_begin): a
+// launch needs nothing before it, and whatever a launch finds in its word, the one after the next
+// starts at 0 again.  A captured launch may be replayed any number of times, beside casts on its stream too: it
+// takes a third word, which a memset node before it zeroes.  Launches on different streams may overlap, so every
+// stream that uses the scene gets words of its own.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -16,27 +18,77 @@
 namespace svo {
 
 constexpr uint32_t kQueueSlots = 64;
+// Words of a stream: two that its launches take in turn, the captured launches' and one that those "zero" for nobody.
+constexpr uint32_t kQueueWords = 4;
+
+// Which of a stream's words its next launch claims from.
+struct QueueTurn {
+  uint32_t turn = 0;
+  uint32_t word(bool captured) const { return captured ? 2u : turn; }
+  void launched(bool captured) {  // it is in the stream, and will zero the other word
+    if (!captured) turn ^= 1u;
+  }
+};
+
+// The claim word of the next launch on the stream of the launch whose word `queue` is: the other of the pair.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline unsigned long long* queue_next(unsigned long long* queue) {
+  return reinterpret_cast<unsigned long long*>(reinterpret_cast<uintptr_t>(queue) ^ sizeof(unsigned long long));
+}
+#ifdef __CUDACC__
+// Zeroes it; no other launch of the stream runs meanwhile.
+__device__ __forceinline__ void queue_begin(unsigned long long* queue) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *queue_next(queue) = 0;
+}
+#endif
 
 struct CastQueues {
   std::mutex m;
   cudaStream_t streams[kQueueSlots] = {};
+  QueueTurn turns[kQueueSlots];
   uint32_t used = 0;
-  unsigned long long* counters = nullptr;  // per slot: claims taken past the warps' own, warps finished
+  unsigned long long* counters = nullptr;  // kQueueSlots * kQueueWords
   int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0, blocks_per_sm_plain = 0;
 };
 
-// The counter of stream `st` (claimed on first use), or nullptr when the scene has none for it:
+// The words of one stream, or of a batch workspace.
+struct QueueWords {
+  unsigned long long* words = nullptr;  // nullptr: none
+  QueueTurn* turn = nullptr;
+};
+
+// The words of stream `st` (claimed on first use), or none where the scene has none for it:
 // all slots taken, or the per-thread default stream, which names a different stream in every
-// host thread.  Call with q->m held.
-inline unsigned long long* queue_counter(CastQueues* q, cudaStream_t st) {
-  if (!q || st == cudaStreamPerThread) return nullptr;
+// host thread.  Call with q->m held until the launch is in the stream.
+inline QueueWords queue_words(CastQueues* q, cudaStream_t st) {
+  if (!q || st == cudaStreamPerThread) return {};
   uint32_t slot = 0;
   while (slot < q->used && q->streams[slot] != st) ++slot;
   if (slot == q->used) {
-    if (q->used == kQueueSlots) return nullptr;
+    if (q->used == kQueueSlots) return {};
     q->streams[q->used++] = st;
   }
-  return q->counters + 2 * slot;
+  return {q->counters + kQueueWords * slot, q->turns + slot};
+}
+
+// One launch's word: `word` goes to the kernel, `launched` follows its launch.
+struct QueueLaunch {
+  unsigned long long* word = nullptr;
+  QueueTurn* turn = nullptr;
+  bool captured = false;
+  void launched() { turn->launched(captured); }
+};
+
+inline cudaError_t queue_take(const QueueWords& q, cudaStream_t st, QueueLaunch& out) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &capturing);
+  out.captured = capturing != cudaStreamCaptureStatusNone;
+  out.turn = q.turn;
+  out.word = q.words + q.turn->word(out.captured);
+  if (e == cudaSuccess && out.captured) e = cudaMemsetAsync(out.word, 0, sizeof(unsigned long long), st);
+  return e;
 }
 
 }  // namespace svo

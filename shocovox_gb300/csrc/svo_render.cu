@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(128, 7)
   const uint64_t warps = (uint64_t)gridDim.x * 4u;
   uint32_t count = 0;  // pixels waiting (the same in every lane)
   unsigned long long t = (uint64_t)blockIdx.x * 4u + (threadIdx.x >> 5);
+  queue_begin(queue);
   bool own = true, more = true;  // the warp's own tile is to take; tiles left
   for (;;) {
     bool have = false, fast = false;
@@ -195,7 +196,6 @@ __global__ void __launch_bounds__(128, 7)
     }
     count_unshaded(bad, unshaded);
   }
-  queue_done(queue, warps);
 }
 
 // One 16 x 8 tile per block (8 x 4 per warp), blockIdx.z the view, for streams without a work counter.
@@ -256,16 +256,19 @@ svo_status render_views(svo_scene* sc, const svo_viewport* vps, uint32_t n_views
   CastQueues* q = sc->dev.queues;
   if (q && tiles < 0xFFFFFFFFull && W < 65536u && H < 65536u) {  // the queue packs a pixel's x and y in 16 bits each
     std::lock_guard<std::mutex> lock(q->m);
-    if (unsigned long long* ctr = queue_counter(q, st)) {
+    if (const QueueWords words = queue_words(q, st); words.words) {
+      QueueLaunch take;
+      SVO_CUDA_TRY(queue_take(words, st, take));
       static const int per_sm = [] {  // resident blocks per SM: the same kernel on every GPU of a process
         int v = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, render_queue_kernel, 128, 0) == cudaSuccess ? v : 1;
       }();
       const uint64_t grid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per_sm, 1), (tiles + 3) / 4);
-      render_queue_kernel<<<(unsigned)grid, 128, 0, st>>>(scene_view(sc), fs, W, H, out, unshaded, ctr, (W + 7) / 8,
+      render_queue_kernel<<<(unsigned)grid, 128, 0, st>>>(scene_view(sc), fs, W, H, out, unshaded, take.word, (W + 7) / 8,
                                                            (uint32_t)tiles_per_view, (uint32_t)tiles,
                                                            pack_target(tiles, (uint64_t)q->sm_count * std::max(per_sm, 1) * 4u));
       SVO_CUDA_TRY(cudaGetLastError());
+      take.launched();
       return SVO_OK;
     }
   }

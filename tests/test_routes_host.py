@@ -1,4 +1,4 @@
-"""The host-side rules of the casts (shocovox_gb300/csrc/svo_route.h), compiled with the host compiler."""
+"""The host-side rules of the casts (shocovox_gb300/csrc/svo_route.h, svo_queue.h), compiled with the host compiler."""
 import ctypes
 import os
 import shutil
@@ -66,3 +66,57 @@ def test_overlap_of_host_arrays(route):
         for off in (-size * n, 4 * n):
             assert not over(**{k: at + off}), (k, off)
         assert not over(0, **{k: at + 4})
+
+
+CLAIMS = 5
+
+
+def test_claim_words_of_a_stream_heal(route):
+    """A stream's launches one after another each start from a claim word that is 0, whatever an overlap of two of them
+    (two streams under one handle) or a replayed graph did before; a captured launch starts from 0 as often as it is replayed."""
+    rng = np.random.default_rng(3)
+
+    class Stream:
+        def __init__(self):
+            self.words, self.turn = [0] * route.route_words(), 0
+
+        def launch(self, captured=False):
+            """The steps of a launch's kernel: what it zeroes, and its claims; returns the word it started from."""
+            w = route.route_word(self.turn, int(captured))
+            self.turn = route.route_launched(self.turn, int(captured))
+            return w
+
+        def steps(self, w, start):
+            """`start`: gets the value the word had at the first claim."""
+            yield self.words.__setitem__(route.route_zeroes(w), 0)
+            start.append(self.words[w])
+            while True:
+                self.words[w] += 1
+                if self.words[w] > CLAIMS:
+                    break
+                yield
+            yield
+
+        def run(self, captured=False):
+            w, start = self.launch(captured), []
+            if captured:
+                self.words[w] = 0  # the graph's memset node
+            for _ in self.steps(w, start):
+                pass
+            return start[0]
+
+    for _ in range(300):
+        s = Stream()
+        for _ in range(rng.integers(0, 4)):
+            assert s.run() == 0
+        # two launches overlap, their steps in any order
+        both = [s.steps(s.launch(), []) for _ in range(2)]
+        while both:
+            k = int(rng.integers(len(both)))
+            if next(both[k], StopIteration) is StopIteration:
+                both.pop(k)
+        s.run()  # the one after them may find a word that one of them was still counting in
+        for _ in range(4):
+            if rng.integers(2):
+                assert s.run(captured=True) == 0
+            assert s.run() == 0
