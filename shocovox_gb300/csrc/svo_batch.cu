@@ -351,6 +351,7 @@ struct svo_batch_workspace {
   svo::BatchItemDev* d_items = nullptr;
   unsigned long long* d_counter = nullptr;  // [0] claim-order work counter, from [2] on the words of the loose items' launches
   svo::QueueTurn turn;
+  bool zeroed = false;  // the words have been zeroed, by the first launch that took one of the pair
   svo::BatchItemDev* h_items = nullptr;     // pinned
   svo::LooseItemDev* d_loose = nullptr;     // the items of batch_flow_kernel
   svo::LooseItemDev* h_loose = nullptr;     // pinned
@@ -370,8 +371,6 @@ svo_status svo_batch_workspace_create(svo_batch_workspace** out) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ws->sm_count, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaMalloc(&ws->d_counter, (2 + kQueueWords) * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(ws->d_counter, 0, (2 + kQueueWords) * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // casts may follow on any stream
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->copied, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     cudaFree(ws->d_counter);
@@ -479,6 +478,10 @@ svo_status svo_cast_batched(svo_batch_workspace* ws, const svo_batch_item* items
     const uint32_t below = refill ? 33u - refill : kFlowRefill;
     QueueLaunch take;
     SVO_CUDA_TRY(queue_take({ws->d_counter + 2, &ws->turn}, st, take));
+    if (!take.captured && !ws->zeroed) {
+      SVO_CUDA_TRY(cudaMemsetAsync(ws->d_counter + 2, 0, 2 * sizeof(unsigned long long), st));
+      ws->zeroed = true;
+    }
     const uint32_t per_sm = cfg ? cfg->blocks_per_sm : 0;
     if (n_loose == 1) {
       const BatchItemDev& d = ws->h_items[one];

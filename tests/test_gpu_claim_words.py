@@ -1,5 +1,7 @@
 """Claim words of the queued casts across launches: graphs replayed beside casts on the stream they were captured on, and
 casts after an overlap that include/svo.h rules out (two graphs of one stream at once), which may spoil those two only."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -102,3 +104,26 @@ def test_casts_after_two_graphs_of_a_stream_overlapped(scene):
             with torch.cuda.stream(s):
                 g.replay()
             c.check("replay %d" % k)
+
+
+def test_workspace_creation_leaves_the_default_stream_alone():
+    """It neither waits for work that the default stream has queued nor ends a capture that the stream must not touch."""
+    svo.BatchWorkspace()
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(400_000_000)  # about 0.2 s
+    busy.record()
+    ws = svo.BatchWorkspace()
+    assert not busy.query()
+    busy.synchronize()
+    rt = ctypes.CDLL("libcudart.so.13")
+    st, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(st)) == 0  # one that the default stream waits for
+    assert rt.cudaStreamBeginCapture(st, 2) == 0  # relaxed: allocations are allowed meanwhile
+    try:
+        other = svo.BatchWorkspace()
+    finally:
+        rc = rt.cudaStreamEndCapture(st, ctypes.byref(graph))
+    assert rc == 0
+    assert rt.cudaGraphDestroy(graph) == 0 and rt.cudaStreamDestroy(st) == 0
+    del ws, other
