@@ -295,20 +295,8 @@ __global__ void __launch_bounds__(128, 6)
                       unsigned long long* __restrict__ queue) {
   __shared__ FlowShared sh;
   __shared__ FlowLists<BatchRayId> lists[4];
-  FlowLists<BatchRayId>& w = lists[threadIdx.x >> 5];
   queue_begin(queue);
-  unsigned long long c = flow_claim(queue);
-  while (uint32_t others = flow_cast(src, claims, refill, queue, c, sh, w)) {
-    for (uint32_t k = threadIdx.x & 31u; k < others; k += 32u) {
-      const BatchRayId id = w.other[k];
-      float o[3], d[3];
-      src.ray(id, o, d);
-      HitRecord h;
-      cast_one<false>(src.scene(id), kLuts, o[0], o[1], o[2], d[0], d[1], d[2], h);
-      src.put(id, h);
-    }
-    __syncwarp();
-  }
+  flow_batch(src, claims, refill, queue, sh, lists[threadIdx.x >> 5]);
 }
 
 }  // namespace svo

@@ -231,20 +231,7 @@ __global__ void __launch_bounds__(128, 6)
     queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
     return;
   }
-  const uint32_t lane = threadIdx.x & 31u;
-  FlowLists<RayId>& lists = m.flow;
-  unsigned long long c = flow_claim(queue);
-  while (uint32_t others = flow_cast(src, src.order.claims, refill, queue, c, sh, lists)) {
-    for (uint32_t k = lane; k < others; k += 32u) {
-      const RayId id = lists.other[k];
-      float o[3], d[3];
-      src.ray(id, o, d);
-      HitRecord h;
-      cast_one<false>(src.s, kLuts, o[0], o[1], o[2], d[0], d[1], d[2], h);
-      src.put(id, h);
-    }
-    __syncwarp();
-  }
+  flow_batch(src, src.order.claims, refill, queue, sh, m.flow);
 }
 
 // Host-buffer cast that reads its rays from and writes its hits to host memory in place (over the CPU

@@ -323,8 +323,8 @@ template <class Id>
 struct FlowLists {
   float p[3][64];
   Id id[64];
-  Id other[64];
-  Id lane[32];  // the lanes' rays
+  Id other[96];  // fewer than 32 wait before a claim; it adds 32 at most, and so do the rays in flight
+  Id lane[32];   // the lanes' rays
   uint8_t target[64];
 };
 
@@ -333,10 +333,10 @@ struct FlowLists {
 //   ray(id, o, d)              its origin and direction
 //   scene(id)                  its scene
 //   put(id, h)                 writes its record
-// c is the warp's next claim, from the counter queue[0] like queue_cast's: whichever of the two a block runs, each
-// claim is cast once.
-// Returns how many rays wait in w.other for the general forms: 0 once the batch is done.  Where there are
-// some the caller casts them and calls again (no ray is in flight then, so their registers are free).
+// c is the warp's next claim, from the counter *queue like queue_cast's: whichever of the two a block runs, each
+// claim is cast once; `count` and `others` rays wait in the lists, none of them at first.
+// Returns once a warp of rays waits for the general forms, or nothing but some of those is left, with no ray in flight
+// (so their registers are free): flow_batch casts them and calls again.
 //
 // Rays that miss the root box get their miss at once, the others wait in the warp's list.  Once
 // kFlowRefill lanes (or `refill`) have no running ray, their records are written and the next listed rays
@@ -353,13 +353,12 @@ __device__ __forceinline__ unsigned long long flow_claim(unsigned long long* __r
 }
 
 template <class Src, class Id>
-__device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, uint32_t refill,
+__device__ __forceinline__ void flow_cast(const Src& src, uint64_t claims, uint32_t refill,
                                               unsigned long long* __restrict__ queue, unsigned long long& c,
-                                              FlowShared& sh, FlowLists<Id>& w) {
+                                              uint32_t& count, uint32_t& others, FlowShared& sh, FlowLists<Id>& w) {
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   uint32_t tid = threadIdx.x;
   asm volatile("" : "+r"(tid));  // kept in a register: each use read the special register again (680 -> 665 us)
-  uint32_t count = 0, others = 0;  // rays in the lists (the same in every lane)
   w.lane[lane] = Id{};
   __syncwarp();
   Flow f{};  // every field set: nothing of a ray lives on from the last call
@@ -385,9 +384,9 @@ __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, u
     others += __popc(g);
     const unsigned idle = __ballot_sync(0xFFFFFFFFu, f.mode == kIdle);
     const uint32_t need = __popc(idle);
-    // claims until every idle lane can have a ray; not past a ray for the general forms, which wait until
-    // the rays in flight have ended
-    while (c < claims && count < need && others == 0u) {
+    // claims until every idle lane can have a ray, or a warp of rays waits for the general forms: those are cast
+    // when the rays in flight have ended
+    while (c < claims && count < need && others < 32u) {
       bool unit = false, other = false;
       float p[3] = {};
       uint32_t target = 0;
@@ -415,13 +414,13 @@ __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, u
         w.target[k] = (uint8_t)target;
         w.id[k] = id;
       }
-      if (other) w.other[__popc(mo & below)] = id;
+      if (other) w.other[others + __popc(mo & below)] = id;
       count += __popc(mu);
-      others = __popc(mo);
+      others += __popc(mo);
       c = flow_claim(queue);
     }
     __syncwarp();
-    const uint32_t take = count < need ? count : need;
+    const uint32_t take = others >= 32u ? 0u : count < need ? count : need;
     if (f.mode == kIdle) {
       const uint32_t k = __popc(idle & below);
       if (k < take) {
@@ -435,8 +434,8 @@ __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, u
     }
     count -= take;
     __syncwarp();
-    const bool left = count > 0 || (c < claims && others == 0u);
-    if (!left && !__any_sync(0xFFFFFFFFu, f.mode != kIdle)) return others;
+    const bool left = others < 32u && (count > 0 || c < claims);
+    if (!left && !__any_sync(0xFFFFFFFFu, f.mode != kIdle)) return;
     // ---- run until `refill` lanes have no running ray (all lanes, once nothing is left to hand out)
     const uint32_t stop = left ? 32u - refill : 0u;
     while (__popc(__ballot_sync(0xFFFFFFFFu, f.mode >= kVisit)) > stop) {
@@ -447,6 +446,31 @@ __device__ __forceinline__ uint32_t flow_cast(const Src& src, uint64_t claims, u
       if (f.mode >= kStep) flow_step(f, s, sh, tid);
       __syncwarp();
     }
+  }
+}
+
+// A batch's rays, all of them.  Rays for the general forms are cast a warp of them at a time (cast a claim's few at a time,
+// as they came, 2^22 random rays on 512^3 of which a tenth are not of unit length took 1,626 us, all of them 1,598).
+template <class Src, class Id>
+__device__ __forceinline__ void flow_batch(const Src& src, uint64_t claims, uint32_t refill,
+                                           unsigned long long* __restrict__ queue, FlowShared& sh, FlowLists<Id>& w) {
+  const uint32_t lane = threadIdx.x & 31u;
+  unsigned long long c = flow_claim(queue);
+  uint32_t count = 0, others = 0;
+  for (;;) {
+    flow_cast(src, claims, refill, queue, c, count, others, sh, w);
+    if (others == 0u) return;
+    const uint32_t take = others < 32u ? others : 32u;
+    others -= take;
+    if (lane < take) {
+      const Id id = w.other[others + lane];
+      float o[3], d[3];
+      src.ray(id, o, d);
+      HitRecord h;
+      cast_one<false>(src.scene(id), kLuts, o[0], o[1], o[2], d[0], d[1], d[2], h);
+      src.put(id, h);
+    }
+    __syncwarp();
   }
 }
 

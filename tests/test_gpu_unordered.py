@@ -1,0 +1,96 @@
+"""The unordered items of a batched cast (svo_launch_config.sort_key = 1) without counters: one item is cast by
+plain_kernel, several by batch_flow_kernel.  (Calls that ask for counters are cast in claim order.)"""
+import numpy as np
+import pytest
+
+import shocovox_gb300 as svo
+from test_gpu_cast import assert_same_hits, both
+from test_gpu_flow import UNCOUNTED, random_rays
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+NOISE = dict(seed=31, occupancy=0.08, spheres=3, octaves=2, base_freq=1.0 / 16, height_lo=2.0, height_hi=24.0)
+
+
+class Items:
+    """Items of one call over (scene, origins, directions, row length); `check` compares them with the oracle."""
+
+    def __init__(self, parts):
+        self.items, self.keep = [], []
+        for (o, p), origins, dirs, row in parts:
+            n = len(origins)
+            cols = {k: torch.from_numpy(np.ascontiguousarray(a[:, i])).cuda()
+                    for a, names in ((origins, ("ox", "oy", "oz")), (dirs, ("dx", "dy", "dz"))) for i, k in enumerate(names)}
+            out = {k: torch.zeros(n + 33, dtype=getattr(torch, np.dtype(svo.HIT_FIELDS[k]).name), device="cuda")
+                   for k in UNCOUNTED}
+            self.items.append((p, {k: v.data_ptr() for k, v in cols.items()}, n, {k: v.data_ptr() for k, v in out.items()}, row))
+            self.keep.append((cols, out, n, o.cast(origins, dirs, threads=16) if n else None))
+
+    def clear(self):
+        for _, out, _, _ in self.keep:
+            for v in out.values():
+                v.fill_(0x5A)
+        torch.cuda.synchronize()
+
+    def check(self, label):
+        torch.cuda.synchronize()
+        for j, (_, out, n, ref) in enumerate(self.keep):
+            got = {k: v.cpu().numpy() for k, v in out.items()}
+            assert all((v[n:] == 0x5A).all() for v in got.values()), "written past item %d" % j
+            if n:
+                assert_same_hits({k: v[:n] for k, v in got.items()}, ref, label="%s item %d" % (label, j))
+
+    def cast(self, ws, cfg, label):
+        self.clear()
+        ws.cast(self.items, cfg, torch.cuda.current_stream().cuda_stream)
+        self.check(label)
+
+
+def spoiled(rng, dirs, share):
+    """Directions of which `share` are not of unit length, so that the general forms cast them."""
+    dirs = dirs.copy()
+    dirs[rng.random(len(dirs)) < share] *= np.float32(1.5)
+    return dirs
+
+
+@pytest.mark.parametrize("share", [0.0, 0.003, 0.05, 0.5, 1.0])
+@pytest.mark.parametrize("n_items", [1, 3])
+def test_rays_for_the_general_forms_among_others(oracle_mod, share, n_items):
+    """They wait in a warp's list until there is a warp of them, or nothing else is left, whatever their share."""
+    rng = np.random.default_rng(int(share * 1000) + n_items)
+    scene = both(oracle_mod, 64, 4, svo.gen_scene(3, 64, 4, **NOISE))
+    parts = []
+    for n in (200_003, 33, 70_001)[:n_items]:
+        origins, dirs = random_rays(rng, 64, n)
+        parts.append((scene, origins, spoiled(rng, dirs, share), 0))
+    items, ws = Items(parts), svo.BatchWorkspace()
+    for refill in (0, 1, 32):
+        items.cast(ws, svo.LaunchConfig(0, 0, 0, 0, 1, 0, refill), "refill %d" % refill)
+    items.cast(ws, svo.LaunchConfig(0, 0, 1, 0, 1, 0, 0), "one block per SM")
+
+
+def test_directions_off_unit_length_cost_about_what_claim_order_costs(oracle_mod):
+    """2^21 rays, all for the general forms: the same forms as in claim order, a warp at a time; 1.3 for two entry tests
+    a ray and 6 blocks per SM instead of 7.  (Cast a claim's few at a time: 1.8.)"""
+    _, p = both(oracle_mod, 256, 8, svo.gen_scene(2, 256, 8, seed=31, occupancy=0.08))
+    n = 1 << 21
+    origins, dirs = svo.gen_sphere_rays([128.0] * 3, 128 * np.sqrt(3.0), n, 5)
+    cols = {k: torch.from_numpy(np.ascontiguousarray(a[:, i] * np.float32(f))).cuda() for a, f, names in
+            ((origins, 1.0, ("ox", "oy", "oz")), (dirs, 1.5, ("dx", "dy", "dz"))) for i, k in enumerate(names)}
+    status = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    item = [(p, {k: v.data_ptr() for k, v in cols.items()}, n, {"status": status.data_ptr()}, 0)]
+    ws = svo.BatchWorkspace()
+
+    def ms(key):
+        times = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ws.cast(item, svo.LaunchConfig(0, 0, 0, 0, key, 0, 0), torch.cuda.current_stream().cuda_stream)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return float(np.median(times[3:]))
+
+    ordered, unordered = ms(0), ms(1)
+    assert unordered < 1.3 * ordered, (unordered, ordered)
