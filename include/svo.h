@@ -297,7 +297,8 @@ typedef struct {
   uint32_t sort_key;       /* the rays of the items without a row length: 0 = cast 32 neighbours at a time,
                               1 = in no particular order: cast a step of each ray at a time, a warp's
                               idle lanes taking new rays (svo_cast_batched only; fewer than 2^32 such
-                              rays per call) */
+                              rays per call; a lone item whose rays keep together all the same, as a sample
+                              of them shows, is cast 32 at a time) */
   uint32_t staging_depth;  /* top tree levels staged in shared memory by every block: the Internal nodes of
                               depth < staging_depth (0..4) of each scene of the call, as far as 48 KB of
                               records per block reach (scenes past that read their nodes from L1/L2) */
@@ -440,10 +441,10 @@ svo_status svo_set_host_transfer(int32_t mode);
  * svo_launch_config.staging_depth.  No counterpart in the reference. */
 svo_status svo_set_staging_depth(int32_t depth);
 /* Lane refill of the plain casts launched afterwards (process-wide): 0 (default) lets large batches
- * without a row layout choose by a sample of their rays; 1..32: every batch of 131,072 rays and more is
- * cast a step of each ray at a time, and a warp whose rays in flight drop below park_below gives its idle
- * lanes new rays, so that rays of very different lengths (rays in no particular order) keep the
- * lanes busy.  The results are the same for every value.  No counterpart in the reference. */
+ * without a row layout choose by a sample of their rays; 1..32: so do all batches of 131,072 rays and
+ * more, and where the rays go their own ways, cast a step of each at a time, a warp whose rays in flight drop below
+ * park_below gives its idle lanes new rays, so that rays of very different lengths keep the lanes busy.
+ * The results are the same for every value.  No counterpart in the reference. */
 svo_status svo_set_refill(int32_t park_below);
 
 #ifdef __cplusplus

@@ -208,8 +208,10 @@ __global__ void __launch_bounds__(128, 7)
   }
 }
 
-// A large batch without a row layout: a camera's rays in raster order, which queue_cast casts, or rays in
-// no order, which flow_cast casts but for those of the general forms.  The rays themselves tell (rays_mixed).
+// A large batch without a row layout, or one that the caller says is in no order: a camera's rays in raster order, or
+// rays for the general forms, which queue_cast casts, or rays in no order, which flow_cast does.  The rays themselves
+// tell (rays_mixed), whatever the caller says: four cameras of 1920 x 1080 on 512^3 take 2,170 to 5,160 us in flow_cast
+// (refill thresholds 1 to 32) and 1,545 in queue_cast, 2^22 random rays not of unit length 917 and 868.
 // Hits may be written over the rays, and a warp that starts late reads some of them: warps may answer differently.  So they
 // share no memory, and both casts take their claims from one counter.
 union PlainLists {  // one warp's
@@ -222,13 +224,13 @@ union PlainLists {  // one warp's
 // Larger camera batches pay for the block that queue_kernel has more: 2.07 M rays 837 us against 826, 8.29 M 3,165 against 3,058.
 __global__ void __launch_bounds__(128, 6)
     plain_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ queue, uint32_t refill,
-                 bool test) {
+                 uint32_t pack) {
   __shared__ FlowShared sh;
   __shared__ PlainLists lists_of[4];
   PlainLists& m = lists_of[threadIdx.x >> 5];
   queue_begin(queue);
-  if (test && !rays_mixed(src.rays, src.n, src.s)) {
-    queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr);
+  if (!rays_mixed(src.rays, src.n, src.s)) {
+    queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr, 0.0f, 0, pack);
     return;
   }
   flow_batch(src, src.order.claims, refill, queue, sh, m.flow);
@@ -890,7 +892,7 @@ uint32_t grid_lanes(uint64_t n) {
 }
 
 }  // namespace
-// plain_kernel over one batch whose rays are in no order (svo_batch.cu).  `queue`: its claim word (svo_queue.h).
+// plain_kernel over one batch said to be in no order (svo_batch.cu).  `queue`: its claim word (svo_queue.h).
 svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView& hits, uint64_t n, uint32_t refill,
                         uint32_t blocks_per_sm, unsigned long long* queue, cudaStream_t st) {
   int dev = 0, sms = 0, per = (int)blocks_per_sm;
@@ -899,7 +901,8 @@ svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView
   if (per == 0) SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, plain_kernel, 128, 0));
   const ClaimOrder order = claim_order(n, 0);
   const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)std::max(per, 1), (order.claims + 3) / 4);
-  plain_kernel<<<(unsigned)grid, 128, 0, st>>>(ArraySource{v, rays, hits, n, order}, queue, refill, false);
+  plain_kernel<<<(unsigned)grid, 128, 0, st>>>(ArraySource{v, rays, hits, n, order}, queue, refill,
+                                               pack_target(order.claims, grid * 4u));
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }
@@ -939,7 +942,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         pair_rows_kernel<<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
       } else if (flow && g_refill_below > 0) {
         plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue,
-                                                             33u - (uint32_t)g_refill_below, false);
+                                                             33u - (uint32_t)g_refill_below, pack);
       } else if (stage_n) {
         // the staged records take dynamic shared memory: resident blocks from this launch's size
         const size_t smem = (size_t)stage_n * sizeof(DevNode);
@@ -954,7 +957,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
       } else if (row || in_place || !flow || n < kFlowMinRays) {
         queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack);
       } else {
-        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, true);
+        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, pack);
       }
       SVO_CUDA_TRY(cudaGetLastError());
       take.launched();

@@ -517,8 +517,9 @@ SVO_UHD uint64_t pair_at(uint64_t n, uint32_t k) {
 }
 
 // Whether neighbouring rays of a batch go their own ways: of 32 pairs of rays, spread over the batch,
-// fewer than 24 head into one octant, within 25 degrees, from origins within an eighth of the octree; and all are
-// of the unit form.  Every warp of a launch reads the same 12 x 32 values and comes to the same answer.
+// fewer than 24 head into one octant, within 25 degrees, from origins within an eighth of the octree; and half of them or
+// more are of the unit form (2^22 random rays on 512^3, a quarter of them not of unit length: 885 us in flow_cast, 979 in
+// queue_cast; 30%: 951, 975; 40%: 1,003, 961).  Every warp of a launch reads the same 12 x 32 values and comes to the same answer.
 __device__ __forceinline__ bool rays_mixed(const RaysView& r, uint64_t n, const SceneView& s) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t a = pair_at(n, lane), b = n <= kPairApart ? n - 1u : a + kPairApart;
@@ -531,7 +532,7 @@ __device__ __forceinline__ bool rays_mixed(const RaysView& r, uint64_t n, const 
                      ax * bx + ay * by + az * bz > 0.9f && fabsf(ux - vx) < near && fabsf(uy - vy) < near &&
                      fabsf(uz - vz) < near;
   const bool unit = unit_eligible(s, ux, uy, uz, ax, ay, az) && unit_eligible(s, vx, vy, vz, bx, by, bz);
-  return __popc(__ballot_sync(0xFFFFFFFFu, along)) < 24 && __all_sync(0xFFFFFFFFu, unit);
+  return __popc(__ballot_sync(0xFFFFFFFFu, along)) < 24 && __popc(__ballot_sync(0xFFFFFFFFu, unit)) >= 16;
 }
 
 }  // namespace svo

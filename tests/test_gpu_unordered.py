@@ -46,6 +46,18 @@ class Items:
         self.check(label)
 
 
+def median_ms(call):
+    times = []
+    for _ in range(12):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        call()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b))
+    return float(np.median(times[3:]))
+
+
 def spoiled(rng, dirs, share):
     """Directions of which `share` are not of unit length, so that the general forms cast them."""
     dirs = dirs.copy()
@@ -81,16 +93,30 @@ def test_directions_off_unit_length_cost_about_what_claim_order_costs(oracle_mod
     item = [(p, {k: v.data_ptr() for k, v in cols.items()}, n, {"status": status.data_ptr()}, 0)]
     ws = svo.BatchWorkspace()
 
-    def ms(key):
-        times = []
-        for _ in range(12):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            ws.cast(item, svo.LaunchConfig(0, 0, 0, 0, key, 0, 0), torch.cuda.current_stream().cuda_stream)
-            b.record()
-            torch.cuda.synchronize()
-            times.append(a.elapsed_time(b))
-        return float(np.median(times[3:]))
-
-    ordered, unordered = ms(0), ms(1)
+    ordered, unordered = (median_ms(lambda: ws.cast(item, svo.LaunchConfig(0, 0, 0, 0, key, 0, 0),
+                                                    torch.cuda.current_stream().cuda_stream)) for key in (0, 1))
     assert unordered < 1.3 * ordered, (unordered, ordered)
+
+
+@pytest.mark.parametrize("row", [0, 1920])
+def test_refill_of_rays_that_keep_together_costs_about_nothing(oracle_mod, row):
+    """A camera's rays are cast 32 neighbours at a time whatever svo_set_refill says; 1.3 for 6 blocks per SM instead of 7 and
+    a look at the rays.  (One step of each at a time: 2.3.)"""
+    _, p = both(oracle_mod, 256, 8, svo.gen_scene(1, 256, 8, seed=77, octaves=3, base_freq=1.0 / 64, height_lo=5.0,
+                                                  height_hi=80.0))
+    origins, dirs = svo.gen_camera_rays([40.0, 120.0, 30.0], [200.0, 20.0, 180.0], 70.0, 1920, 1080)
+    n = len(origins)
+    cols = {k: torch.from_numpy(np.ascontiguousarray(a[:, i])).cuda()
+            for a, names in ((origins, ("ox", "oy", "oz")), (dirs, ("dx", "dy", "dz"))) for i, k in enumerate(names)}
+    status = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    rays, hits = {k: v.data_ptr() for k, v in cols.items()}, {"status": status.data_ptr()}
+
+    def ms(refill):
+        svo.check(svo.lib().svo_set_refill(refill))
+        try:
+            return median_ms(lambda: p.cast(rays, hits, n, torch.cuda.current_stream().cuda_stream, row))
+        finally:
+            svo.lib().svo_set_refill(0)
+
+    off, on = ms(0), ms(24)
+    assert on < 1.3 * off, (on, off)
