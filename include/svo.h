@@ -214,7 +214,8 @@ svo_status svo_set_device_allocator(svo_alloc_fn alloc, svo_free_fn release, voi
  * Batches of 131,072 rays and more run as a work queue: warps claim 32 rays at a time from a
  * counter that the scene keeps per stream (up to 64 streams; casts on further streams, and on
  * cudaStreamPerThread, use one thread per ray).  From 524,288 rays on, rays without a row layout that
- * go their own ways (a sample of them is looked at on the device) are cast a step of each at a time.  Casts of one scene on different streams may
+ * go their own ways (a sample of them is looked at on the device) are cast a step of each at a time (from 2,621,440
+ * on in a launch apart: one of the two ends at once).  Casts of one scene on different streams may
  * overlap.  A CUDA graph that captured a cast uses a counter of the stream it was captured on: do not run it
  * concurrently with itself, or with another graph captured on that stream (the hits of those two casts would be
  * incomplete, later ones' not). */
@@ -297,8 +298,8 @@ typedef struct {
   uint32_t sort_key;       /* the rays of the items without a row length: 0 = cast 32 neighbours at a time,
                               1 = in no particular order: cast a step of each ray at a time, a warp's
                               idle lanes taking new rays (svo_cast_batched only; fewer than 2^32 such
-                              rays per call; a lone item whose rays keep together all the same, as a sample
-                              of them shows, is cast 32 at a time) */
+                              rays per call; a lone item of 131,072 rays and more that keep together all the
+                              same, as a sample of them shows, is cast 32 at a time) */
   uint32_t staging_depth;  /* top tree levels staged in shared memory by every block: the Internal nodes of
                               depth < staging_depth (0..4) of each scene of the call, as far as 48 KB of
                               records per block reach (scenes past that read their nodes from L1/L2) */

@@ -192,9 +192,11 @@ __device__ __forceinline__ void queue_cast(const SceneView& s, const RaysView& r
 template <bool kCount, bool kLod = false, bool kStage = false>
 __global__ void __launch_bounds__(128, 7)
     queue_kernel(const __grid_constant__ SceneView s, RaysView rays, HitsView out, uint64_t n, ClaimOrder order,
-                 unsigned long long* __restrict__ queue, float viewing_distance, uint32_t stage_n, uint32_t pack) {
+                 unsigned long long* __restrict__ queue, float viewing_distance, uint32_t stage_n, uint32_t pack,
+                 const unsigned long long* __restrict__ mixed) {
   __shared__ WaitingRays waiting[4];
   queue_begin(queue);
+  if (mixed && *mixed) return;  // flow_kernel casts the batch
   if constexpr (kStage) {
     __shared__ SharedLuts L;
     extern __shared__ uint4 staged_smem[];
@@ -209,8 +211,8 @@ __global__ void __launch_bounds__(128, 7)
 }
 
 // A large batch without a row layout, or one that the caller says is in no order: a camera's rays in raster order, or
-// rays for the general forms, which queue_cast casts, or rays in no order, which flow_cast does.  The rays themselves
-// tell (rays_mixed), whatever the caller says: four cameras of 1920 x 1080 on 512^3 take 2,170 to 5,160 us in flow_cast
+// rays for the general forms, which queue_cast casts, or rays in no order, which flow_cast does.  With `look` the rays
+// themselves tell (rays_mixed), whatever the caller says: four cameras of 1920 x 1080 on 512^3 take 2,170 to 5,160 us in flow_cast
 // (refill thresholds 1 to 32) and 1,545 in queue_cast, 2^22 random rays not of unit length 917 and 868.
 // Hits may be written over the rays, and a warp that starts late reads some of them: warps may answer differently.  So they
 // share no memory, and both casts take their claims from one counter.
@@ -219,21 +221,34 @@ union PlainLists {  // one warp's
   WaitingRays waiting;
   __device__ PlainLists() {}
 };
-// 6 blocks per SM (80 registers): at 7 both casts' loops spill, and a camera's 925 K rays on 256^3 take 256 us
-// instead of 241 (243 in queue_kernel's own launch), 2^22 random rays on 512^3 642 us instead of 679.
-// Larger camera batches pay for the block that queue_kernel has more: 2.07 M rays 837 us against 826, 8.29 M 3,165 against 3,058.
+// 6 blocks per SM (80 registers): at 7 the casts, together in one kernel, spill.  Larger batches have a launch for each cast (kTwoCastsMinRays).
 __global__ void __launch_bounds__(128, 6)
     plain_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ queue, uint32_t refill,
-                 uint32_t pack) {
+                 uint32_t pack, bool look) {
   __shared__ FlowShared sh;
   __shared__ PlainLists lists_of[4];
   PlainLists& m = lists_of[threadIdx.x >> 5];
   queue_begin(queue);
-  if (!rays_mixed(src.rays, src.n, src.s)) {
+  if (look && !rays_mixed(src.rays, src.n, src.s)) {
     queue_cast<false>(src.s, src.rays, src.out, src.n, src.order, queue, kLuts, m.waiting, nullptr, 0.0f, 0, pack);
     return;
   }
   flow_batch(src, src.order.claims, refill, queue, sh, m.flow);
+}
+
+// The same for the largest batches: order_kernel tells the rays' order, and of the two launches after it, queue_kernel and
+// flow_kernel, the other one ends at once.  Alone, each of the two casts fits 7 blocks per SM.
+__global__ void __launch_bounds__(32) order_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ mixed) {
+  const bool m = rays_mixed(src.rays, src.n, src.s);
+  if (threadIdx.x == 0) *mixed = m ? 1 : 0;
+}
+__global__ void __launch_bounds__(128, 7)
+    flow_kernel(const __grid_constant__ ArraySource src, unsigned long long* __restrict__ queue, uint32_t refill,
+                const unsigned long long* __restrict__ mixed) {
+  __shared__ FlowShared sh;
+  __shared__ FlowLists<RayId> lists[4];
+  if (!*mixed) return;  // queue_kernel has cast the batch
+  flow_batch(src, src.order.claims, refill, queue, sh, lists[threadIdx.x >> 5]);
 }
 
 // Host-buffer cast that reads its rays from and writes its hits to host memory in place (over the CPU
@@ -332,6 +347,10 @@ constexpr uint64_t kQueueMinRays = 1u << 17;
 // Below this many rays, of which a fifth may enter the octree, too few are left per warp for flow_cast: random rays
 // on 256^3 take 125 us instead of 117 at 320,000, 164 instead of 166 at 640,000, 216 instead of 243 at 1,280,000.
 constexpr uint64_t kFlowMinRays = 1u << 19;
+// From this many rays on plain_kernel's one block per SM less costs more than two launches: on 512^3 4.2 M camera rays take
+// 969 us in plain_kernel, 919 in launches of their own, 8.4 M 1,698 and 1,597, 8.4 M random ones 772 and 738; at 2.1 M both take
+// 571, 302 and 313 for random ones.
+constexpr uint64_t kTwoCastsMinRays = 5u << 19;
 
 void destroy_queues(DeviceImage& d) {
   if (!d.queues) return;
@@ -351,6 +370,7 @@ svo_status create_queues(DeviceImage& d, cudaStream_t st) {
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_count, queue_kernel<true>, 128, 0);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_plain, plain_kernel, 128, 0);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q->blocks_per_sm_flow, flow_kernel, 128, 0);
   if (e == cudaSuccess) e = cudaMalloc(&q->counters, bytes);
   if (e == cudaSuccess) e = cudaMemsetAsync(q->counters, 0, bytes, st);
   if (e != cudaSuccess) {
@@ -892,7 +912,7 @@ uint32_t grid_lanes(uint64_t n) {
 }
 
 }  // namespace
-// plain_kernel over one batch said to be in no order (svo_batch.cu).  `queue`: its claim word (svo_queue.h).
+// plain_kernel over one batch said to be in no order (svo_batch.cu), below the work queue's size without a look at it.  `queue`: its claim word (svo_queue.h).
 svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView& hits, uint64_t n, uint32_t refill,
                         uint32_t blocks_per_sm, unsigned long long* queue, cudaStream_t st) {
   int dev = 0, sms = 0, per = (int)blocks_per_sm;
@@ -902,7 +922,7 @@ svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView
   const ClaimOrder order = claim_order(n, 0);
   const uint64_t grid = std::min<uint64_t>((uint64_t)sms * (uint64_t)std::max(per, 1), (order.claims + 3) / 4);
   plain_kernel<<<(unsigned)grid, 128, 0, st>>>(ArraySource{v, rays, hits, n, order}, queue, refill,
-                                               pack_target(order.claims, grid * 4u));
+                                               pack_target(order.claims, grid * 4u), n >= kQueueMinRays);
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }
@@ -942,7 +962,7 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         pair_rows_kernel<<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue);
       } else if (flow && g_refill_below > 0) {
         plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue,
-                                                             33u - (uint32_t)g_refill_below, pack);
+                                                             33u - (uint32_t)g_refill_below, pack, true);
       } else if (stage_n) {
         // the staged records take dynamic shared memory: resident blocks from this launch's size
         const size_t smem = (size_t)stage_n * sizeof(DevNode);
@@ -951,13 +971,19 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         int per = 0;
         SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, block, smem));
         const uint64_t sgrid = std::min<uint64_t>((uint64_t)q->sm_count * std::max(per, 1), (order.claims + 3) / 4);
-        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n, pack);
+        kern<<<(unsigned)sgrid, block, smem, st>>>(v, rv, hv, n, order, queue, 0.0f, stage_n, pack, nullptr);
       } else if (count) {
-        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack);
+        queue_kernel<true><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack, nullptr);
       } else if (row || in_place || !flow || n < kFlowMinRays) {
-        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack);
+        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack, nullptr);
+      } else if (n < kTwoCastsMinRays) {
+        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, pack, true);
       } else {
-        plain_kernel<<<(unsigned)plain_grid, block, 0, st>>>(ArraySource{v, rv, hv, n, order}, queue, kFlowRefill, pack);
+        const ArraySource src{v, rv, hv, n, order};
+        order_kernel<<<1, 32, 0, st>>>(src, take.mixed);
+        queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack, take.mixed);
+        flow_kernel<<<(unsigned)((uint64_t)q->sm_count * std::max(1, q->blocks_per_sm_flow)), block, 0, st>>>(src, queue, kFlowRefill,
+                                                                                                              take.mixed);
       }
       SVO_CUDA_TRY(cudaGetLastError());
       take.launched();
@@ -1242,9 +1268,9 @@ svo_status svo_cast_lod_rows(svo_scene* sc, const svo_rays* rays, uint64_t n, ui
   QueueLaunch take;
   SVO_CUDA_TRY(queue_take(words, st, take));
   if (count)
-    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack);
+    queue_kernel<true, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack, nullptr);
   else
-    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack);
+    queue_kernel<false, true><<<(unsigned)grid, 128, 0, st>>>(v, rv, hv, n, order, take.word, viewing_distance, 0, pack, nullptr);
   SVO_CUDA_TRY(cudaGetLastError());
   take.launched();
   return SVO_OK;

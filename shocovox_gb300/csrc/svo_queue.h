@@ -6,7 +6,7 @@
 // launch needs nothing before it, and whatever a launch finds in its word, the one after the next
 // starts at 0 again.  A captured launch may be replayed any number of times, beside casts on its stream too: it
 // takes a third word, which a memset node before it zeroes.  Launches on different streams may overlap, so every
-// stream that uses the scene gets words of its own.
+// stream that uses the scene gets words of its own.  Two more say which of two launches is to cast a batch.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,8 +18,9 @@
 namespace svo {
 
 constexpr uint32_t kQueueSlots = 64;
-// Words of a stream: two that its launches take in turn, the captured launches' and one that those "zero" for nobody.
-constexpr uint32_t kQueueWords = 4;
+// Words of a stream: two that its launches take in turn, the captured launches' and one that those "zero" for nobody,
+// and what order_kernel found, captured launches apart from others.
+constexpr uint32_t kQueueWords = 6;
 
 // Which of a stream's words its next launch claims from.
 struct QueueTurn {
@@ -50,7 +51,7 @@ struct CastQueues {
   QueueTurn turns[kQueueSlots];
   uint32_t used = 0;
   unsigned long long* counters = nullptr;  // kQueueSlots * kQueueWords
-  int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0, blocks_per_sm_plain = 0;
+  int sm_count = 0, blocks_per_sm = 0, blocks_per_sm_count = 0, blocks_per_sm_plain = 0, blocks_per_sm_flow = 0;
 };
 
 // The words of one stream, or of a batch workspace.
@@ -76,6 +77,7 @@ inline QueueWords queue_words(CastQueues* q, cudaStream_t st) {
 // One launch's word: `word` goes to the kernel, `launched` follows its launch.
 struct QueueLaunch {
   unsigned long long* word = nullptr;
+  unsigned long long* mixed = nullptr;
   QueueTurn* turn = nullptr;
   bool captured = false;
   void launched() { turn->launched(captured); }
@@ -87,6 +89,7 @@ inline cudaError_t queue_take(const QueueWords& q, cudaStream_t st, QueueLaunch&
   out.captured = capturing != cudaStreamCaptureStatusNone;
   out.turn = q.turn;
   out.word = q.words + q.turn->word(out.captured);
+  out.mixed = q.words + (out.captured ? 5 : 4);
   if (e == cudaSuccess && out.captured) e = cudaMemsetAsync(out.word, 0, sizeof(unsigned long long), st);
   return e;
 }
