@@ -406,7 +406,7 @@ int g_pair_rows = 1;      // host buffers read and written in place: 32 x 2 bloc
 // a node's record and its heads, one per direction octant
 constexpr uint64_t kNodeBytes = sizeof(DevNode) + kHeadPlanes * sizeof(uint4);
 
-// The heads of all node records, one thread per node and plane.  Bound by its traffic (64 bytes in, 128
+// The heads of n node records, one thread per node and plane.  Bound by its traffic (64 bytes in, 128
 // out per node); the records are read once from DRAM, the other planes' reads hit L2.
 __global__ void __launch_bounds__(256) build_heads(const DevNode* __restrict__ nodes, uint32_t n,
                                                    uint4* __restrict__ heads, uint32_t stride) {
@@ -470,11 +470,11 @@ uint32_t staged_records(const svo_scene* sc, uint32_t depth) {
 
 namespace {
 
-// Writes the heads of the image's first `nn` nodes on st, after their records' copies.
-svo_status write_heads(DeviceImage& d, uint64_t nn, cudaStream_t st) {
-  if (nn == 0) return SVO_OK;
-  build_heads<<<dim3((unsigned)((nn + 255) / 256), kHeadPlanes), 256, 0, st>>>(d.nodes, (uint32_t)nn, d.heads,
-                                                                               (uint32_t)d.node_cap);
+// Writes the heads of the image's nodes [first, end) on st, after their records' copies.
+svo_status write_heads(DeviceImage& d, uint64_t first, uint64_t end, cudaStream_t st) {
+  if (first >= end) return SVO_OK;
+  build_heads<<<dim3((unsigned)((end - first + 255) / 256), kHeadPlanes), 256, 0, st>>>(
+      d.nodes + first, (uint32_t)(end - first), d.heads + first, (uint32_t)d.node_cap);
   SVO_CUDA_TRY(cudaGetLastError());
   return SVO_OK;
 }
@@ -721,7 +721,7 @@ svo_status upload_block(svo_scene* sc, cudaStream_t st, bool fill) {
   if (!d.blob_done) SVO_CUDA_TRY(cudaEventCreateWithFlags(&d.blob_done, cudaEventDisableTiming));
   SVO_CUDA_TRY(cudaEventRecord(d.blob_done, st));
   {
-    const svo_status rc = write_heads(d, t.nodes(), st);
+    const svo_status rc = write_heads(d, 0, t.nodes(), st);
     if (rc != SVO_OK) return rc;
   }
   image_synced(t, d);
@@ -800,7 +800,7 @@ svo_status full_upload(svo_scene* sc, cudaStream_t st, bool ordered = false) {
   }
   SVO_CUDA_TRY(cudaMemcpyAsync(d.nodes, d.host_nodes.data(), nn * sizeof(DevNode), cudaMemcpyHostToDevice, st));
   {
-    const svo_status hs = write_heads(d, nn, st);
+    const svo_status hs = write_heads(d, 0, nn, st);
     if (hs != SVO_OK) return hs;
   }
   {
@@ -843,6 +843,10 @@ svo_status copy_runs(std::vector<uint8_t>& flags, uint64_t limit, F&& copy) {
   return SVO_OK;
 }
 
+// Changed nodes fewer than this apart have their heads written by one launch: the heads of the nodes between them
+// (192 bytes of traffic each) take less than another launch.
+constexpr uint64_t kHeadsGap = 1u << 16;
+
 svo_status incremental_sync(svo_scene* sc, cudaStream_t st) {
   HostOctree& t = sc->tree;
   DeviceImage& d = sc->dev;
@@ -863,16 +867,17 @@ svo_status incremental_sync(svo_scene* sc, cudaStream_t st) {
   } catch (const ReferencePanic& p) {
     return fail(SVO_ERR_REFERENCE_PANIC, std::string("sync: ") + p.what());
   }
-  const bool nodes_changed = std::find(t.node_dirty.begin(), t.node_dirty.end(), 1) != t.node_dirty.end();
+  Spans spans;
   svo_status rc = copy_runs(t.node_dirty, nn, [&](uint64_t a, uint64_t b) -> svo_status {
+    add_span(spans, a, b, kHeadsGap);
     SVO_CUDA_TRY(cudaMemcpyAsync(d.nodes + a, d.host_nodes.data() + a, (b - a) * sizeof(DevNode),
                                  cudaMemcpyHostToDevice, st));
     return SVO_OK;
   });
-  if (rc != SVO_OK) return rc;
-  if (nodes_changed) {
-    rc = write_heads(d, nn, st);
-    if (rc != SVO_OK) return rc;
+  for (size_t k = 0; k < spans.size() && rc == SVO_OK; ++k) rc = write_heads(d, spans[k].first, spans[k].second, st);
+  if (rc != SVO_OK) {  // the next sync has to write them all
+    for (const auto& s : spans) std::fill(t.node_dirty.begin() + s.first, t.node_dirty.begin() + s.second, 1);
+    return rc;
   }
   rc = upload_top(d, st);
   if (rc != SVO_OK) return rc;

@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstdint>
+#include <utility>
+#include <vector>
 
 #include "svo_internal.h"
 
@@ -34,6 +36,15 @@ inline bool hits_over_rays(const svo_rays& rays, const svo_hits& hits, uint64_t 
     }
   }
   return false;
+}
+
+// Spans [a, b) of elements, added in order; those fewer than `gap` apart become one.
+using Spans = std::vector<std::pair<uint64_t, uint64_t>>;
+inline void add_span(Spans& spans, uint64_t a, uint64_t b, uint64_t gap) {
+  if (spans.empty() || a - spans.back().second >= gap)
+    spans.push_back({a, b});
+  else
+    spans.back().second = b;
 }
 
 }  // namespace svo

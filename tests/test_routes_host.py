@@ -120,3 +120,26 @@ def test_claim_words_of_a_stream_heal(route):
             if rng.integers(2):
                 assert s.run(captured=True) == 0
             assert s.run() == 0
+
+
+@pytest.mark.parametrize("gap", [1, 2, 7, 65536])
+def test_spans_of_changed_nodes(route, gap):
+    """All runs and nothing else but what lies between runs fewer than `gap` apart."""
+    rng = np.random.default_rng(gap)
+    for case in range(200):
+        ends = np.sort(rng.choice(400, 2 * int(rng.integers(0, 30)), replace=False)).astype(np.uint64)
+        runs = np.ascontiguousarray(ends.reshape(-1, 2))
+        out = np.zeros((len(runs) + 1, 2), np.uint64)
+        k = route.route_spans(runs.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(len(runs)), ctypes.c_uint64(gap),
+                              out.ctypes.data_as(ctypes.c_void_p))
+        covered = np.zeros(400, bool)
+        for a, b in runs.tolist():
+            covered[a:b] = True
+        at = np.nonzero(covered)[0].tolist()
+        expected = []
+        for i in at:
+            if expected and i - expected[-1][1] < gap:
+                expected[-1][1] = i + 1
+            else:
+                expected.append([i, i + 1])
+        assert out[:k].tolist() == expected, case
