@@ -40,8 +40,9 @@ struct BatchItemDev {
 
 constexpr uint32_t kBatchStageRecords = 768;  // 48 KB of staged records per block at most
 
-// Shares the staged records out among the scenes of a call, in order of first appearance, at staging
-// depth `depth` while they fit kBatchStageRecords; returns the records a block copies.
+// Shares the staged records out among the scenes of a call's items in claim order (the others' kernel stages nothing),
+// in order of first appearance, at staging depth `depth` while they fit kBatchStageRecords; returns the
+// records a block copies.
 inline uint32_t assign_staging(BatchItemDev* table, const svo_batch_item* items, uint32_t n_items, uint32_t depth) {
   uint32_t total = 0;
   for (uint32_t i = 0; i < n_items; ++i) {
@@ -51,9 +52,10 @@ inline uint32_t assign_staging(BatchItemDev* table, const svo_batch_item* items,
   }
   if (depth == 0) return 0;
   for (uint32_t i = 0; i < n_items; ++i) {
+    if (table[i].n == 0) continue;
     uint32_t first = i;
     for (uint32_t j = 0; j < i; ++j)
-      if (items[j].scene == items[i].scene) {
+      if (table[j].n != 0 && items[j].scene == items[i].scene) {
         first = j;
         break;
       }
@@ -81,7 +83,7 @@ __device__ __forceinline__ void stage_items(DevNode* stg, const BatchItemDev* it
 }
 
 // fills the device form of one item at global index `begin`; returns the indices it spans
-// (none when the item's rays are cast through the ray sort instead: `claimed` false)
+// (none when the item's rays are cast by batch_flow_kernel instead: `claimed` false)
 uint64_t item_dev(const svo_batch_item& it, uint64_t begin, uint32_t shape, BatchItemDev& d, bool claimed = true) {
   d.scene = scene_view(it.scene);
   d.rays = RaysView{it.rays.ox, it.rays.oy, it.rays.oz, it.rays.dx, it.rays.dy, it.rays.dz};
