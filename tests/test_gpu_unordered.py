@@ -5,6 +5,7 @@ import pytest
 
 import shocovox_gb300 as svo
 from test_gpu_cast import assert_same_hits, both
+from test_gpu_cast import random_rays as special_rays
 from test_gpu_flow import UNCOUNTED, random_rays
 
 pytestmark = pytest.mark.gpu
@@ -120,3 +121,62 @@ def test_refill_of_rays_that_keep_together_costs_about_nothing(oracle_mod, row):
 
     off, on = ms(0), ms(24)
     assert on < 1.3 * off, (on, off)
+
+
+def odd_items(oracle_mod, seed):
+    """Scenes of several sizes and brick dimensions, with empty and 1-ray items, a remainder, and items in claim order."""
+    rng = np.random.default_rng(seed)
+    parts = []
+    for j, (kind, size, dim, n, row) in enumerate([(0, 128, 4, 6000, 0), (3, 64, 2, 1, 0), (3, 32, 8, 0, 0), (1, 64, 8, 33, 0),
+                                                   (2, 256, 8, 20000, 0), (3, 64, 1, 2500, 40), (0, 64, 4, 3000, 0),
+                                                   (3, 64, 4, 0, 0), (3, 64, 4, 3200, 64), (3, 32, 8, 0, 0)]):
+        scene = both(oracle_mod, size, dim, svo.gen_scene(kind, size, dim, seed=seed + j, occupancy=0.1, spheres=3, octaves=2,
+                                                          base_freq=1.0 / 16, height_lo=2.0, height_hi=size * 0.4))
+        origins, dirs = special_rays(rng, size, n)
+        parts.append((scene, origins, dirs, row))
+    return parts
+
+
+@pytest.fixture
+def cast_mode():
+    yield lambda mode: svo.check(svo.lib().svo_set_cast_mode(mode))
+    svo.lib().svo_set_cast_mode(0)
+
+
+def test_several_items(oracle_mod, cast_mode):
+    """Every launch configuration, both cast modes, two calls in a row; an item alone; no unordered item at all."""
+    parts = odd_items(oracle_mod, 700)
+    ws = svo.BatchWorkspace()
+    for mode in (0, 1):
+        cast_mode(mode)
+        items = Items(parts)
+        for cfg in ((0, 0, 0, 0, 1, 0, 0), (64, 32, 0, 0, 1, 2, 1), (128, 100, 0, 4, 1, 0, 8), (96, 256, 3, 0, 1, 4, 32),
+                    (32, 64, 1, 5, 1, 0, 24)):
+            for again in range(2):
+                items.cast(ws, svo.LaunchConfig(*cfg), "mode %d, %s, call %d" % (mode, cfg, again))
+        for only in ([4], [1], [2, 3], [5, 8], [2, 7, 9], [6, 0]):
+            Items([parts[k] for k in only]).cast(ws, svo.LaunchConfig(0, 0, 0, 0, 1, 0, 0), "mode %d, items %s" % (mode, only))
+
+
+def test_workspace_grows_between_calls_and_before_a_graph(oracle_mod):
+    parts = odd_items(oracle_mod, 900)
+    small, large = Items(parts[:1]), Items((parts * 3)[:25])
+    ws, cfg = svo.BatchWorkspace(), svo.LaunchConfig(0, 0, 0, 0, 1, 0, 0)
+    for items, label in ((small, "small"), (large, "grown"), (small, "small again")):
+        items.cast(ws, cfg, label)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ws.cast(large.items, cfg, stream.cuda_stream)
+    for k in range(3):
+        large.clear()
+        graph.replay()
+        large.check("replay %d" % k)
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 31, 32, 33, 40, 41, 127, 129, 131071, 131072])
+def test_sizes_of_a_lone_item(oracle_mod, n):
+    scene = both(oracle_mod, 64, 4, svo.gen_scene(3, 64, 4, **NOISE))
+    ws = svo.BatchWorkspace()
+    camera = tuple(a[:n] for a in svo.gen_camera_rays([150.0, 90.0, 140.0], [32.0, 16.0, 32.0], 50.0, 431, 331))
+    for label, (origins, dirs) in (("random", random_rays(np.random.default_rng(n), 64, n)), ("camera", camera)):
+        Items([(scene, origins, dirs, 0)]).cast(ws, svo.LaunchConfig(0, 0, 0, 0, 1, 0, 0), "%s %d" % (label, n))
