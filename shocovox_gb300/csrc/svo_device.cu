@@ -987,8 +987,12 @@ svo_status launch_cast(svo_scene* sc, const svo_rays* rays, uint64_t n, const sv
         const ArraySource src{v, rv, hv, n, order};
         order_kernel<<<1, 32, 0, st>>>(src, take.mixed);
         queue_kernel<false><<<(unsigned)grid, block, 0, st>>>(v, rv, hv, n, order, queue, 0.0f, 0, pack, take.mixed);
+        SVO_CUDA_TRY(cudaGetLastError());
+        take.launched();  // whether or not the next launch can be made
         flow_kernel<<<(unsigned)((uint64_t)q->sm_count * std::max(1, q->blocks_per_sm_flow)), block, 0, st>>>(src, queue, kFlowRefill,
                                                                                                               take.mixed);
+        SVO_CUDA_TRY(cudaGetLastError());
+        return SVO_OK;
       }
       SVO_CUDA_TRY(cudaGetLastError());
       take.launched();
