@@ -342,6 +342,12 @@ def cast_launches(items, sort_key):
     return (1 if any(it[2] and it not in loose for it in items) else 0) + (1 if loose else 0)
 
 
+def plain_launches(n, row, refill=0, staging=0):
+    """Kernel launches of one svo_cast_rows call: one, but for large batches without rows, whose order one launch tells
+    and which one of two others casts (kTwoCastsMinRays in svo_device.cu; the counted cast is one launch)."""
+    return 3 if not row and n >= 5 << 19 and not refill and not staging else 1
+
+
 def batched_launches(items, sort_key):
     """The launches of the same call while sort_key 1 sorted the rays (bin, three scans, scatter, cast), which
     records of that time count in."""
@@ -617,7 +623,7 @@ def run_single(args, w, workload):
         "cpu_baseline": cpu,
         "e2e": {"value": round(e2e_value, 3), "unit": "Mrays/s", "h2d_bytes_per_step": n * 24,
                 "d2h_bytes_per_step": n * sum(OUT_BYTES.values()), "paths": e2e_paths},
-        "gpu_launches": args.steps,
+        "gpu_launches": args.steps * plain_launches(n, row, args.refill, args.staging_depth),
         "clocks": clk,
         "variants": variants,
         "parity": parity,

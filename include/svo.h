@@ -291,7 +291,8 @@ typedef struct {
 
 typedef struct {
   uint32_t block;          /* threads per block (multiple of 32, <= 128); 0 = default 128 */
-  uint32_t rays_per_chunk; /* rays a warp claims per work-queue grab; 0 = default 64 */
+  uint32_t rays_per_chunk; /* rays a warp claims per work-queue grab; 0 = 64, or 32 where a warp of a full GPU
+                              would claim fewer than 8 times */
   uint32_t blocks_per_sm;  /* persistent CTAs per SM; 0 = default from occupancy */
   uint32_t block_shape;    /* rays of an item with a row length cast together: 0 or 3 = 8 x 4, 4 = 16 x 2,
                               5 = 32 x 1 (log2 of the width) */
@@ -299,7 +300,9 @@ typedef struct {
                               1 = in no particular order: cast a step of each ray at a time, a warp's
                               idle lanes taking new rays (svo_cast_batched only; fewer than 2^32 such
                               rays per call; a lone item of 131,072 rays and more that keep together all the
-                              same, as a sample of them shows, is cast 32 at a time) */
+                              same, as a sample of them shows, is cast 32 at a time).  Such rays have a launch of their own,
+                              which takes blocks_per_sm and refill_below: block is 128, rays_per_chunk 32
+                              and staging_depth 0 there */
   uint32_t staging_depth;  /* top tree levels staged in shared memory by every block: the Internal nodes of
                               depth < staging_depth (0..4) of each scene of the call, as far as 48 KB of
                               records per block reach (scenes past that read their nodes from L1/L2) */

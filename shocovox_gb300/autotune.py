@@ -5,9 +5,11 @@ batches with camera images (items with a row length) the shape of the ray
 blocks a warp casts together, and for batches with rays in no particular order
 (items without a row length) the sort key, on the caller's own batch; then,
 for the fastest of those, the staging depth (top tree levels every block copies
-into shared memory) and, with sort key 1, the lane-refill threshold.  Keeps the fastest and caches the choice per (GPU name,
-workload signature) in a JSON file next to the built library, so later runs skip
-the sweep.
+into shared memory) and, with sort key 1, the lane-refill threshold.  Block size,
+rays per grab and staging depth are the claim-order launch's: a batch of unordered
+items alone takes the same time at all of them.  Keeps the fastest and caches the
+choice per (GPU name, workload signature) in a JSON file next to the built library,
+so later runs skip the sweep.
 """
 import json
 import os
@@ -71,8 +73,7 @@ def tune(ws, items, gpu_name, time_fn, use_cache=True):
         table["%dx%dx%dx%dx%dx%dx0" % (b, c, p, sh, so, st)] = time_fn(_lib.LaunchConfig(b, c, p, sh, so, st, 0))
     if so == 1:
         # sort key 1: its lane-refill threshold at the best staging depth, for every block size (each
-        # with its best rays per claim): the refilling kernel's occupancy is not the plain kernel's, so the
-        # best block without refill need not be the best with it
+        # with its best rays per claim), which matters where items in claim order are cast as well
         st = int(min((k for k in table if k.startswith("%dx%dx%dx%dx%dx" % (b, c, p, sh, so))), key=table.get).split("x")[5])
         for bb in BLOCKS:
             cc = int(min((k for k in table if k.startswith("%dx" % bb) and k.endswith("x%dx%dx%dx0x0" % (p, sh, so))),

@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 7)
 //
 // The items without a row length are cast by flow_cast (svo_flow.cuh), 32 consecutive rays of an item per
 // claim.  It keeps a warp's lanes busy with rays that have nothing in common, so putting like rays into one
-// warp first no longer pays: binning, scanning and scattering 2^20 rays took 60 us, and the sorted cast 300;
-// in index order flow_cast takes 265 in all (GB300, 512^3, 17% entering; 20,000 rays 100 us, 198 before).
+// warp first does not pay: binning, scanning and scattering 2^20 rays took 60 us, and the cast of the sorted
+// rays 300; in index order flow_cast takes 260 in all (GB300, 512^3, 17% entering; 20,000 rays 90 us, 198 sorted).
 struct LooseItemDev {
   uint64_t begin;  // the item's first claim
   uint64_t n;      // its rays (0: the item is cast in claim order)
@@ -568,7 +568,7 @@ svo_status svo_cast_batched_noalloc(const svo_batch_item* items, uint32_t n_item
   if (shape < 3 || shape > 5)
     return fail(SVO_ERR_ARGUMENT, "svo_cast_batched_noalloc: block_shape must be 0, 3, 4 or 5");
   if (cfg && cfg->sort_key)
-    return fail(SVO_ERR_ARGUMENT, "svo_cast_batched_noalloc: the ray sort (sort_key) needs a batch workspace");
+    return fail(SVO_ERR_ARGUMENT, "svo_cast_batched_noalloc: sort_key 1 needs a batch workspace");
   uint64_t total = 0;
   bool count = false;
   for (uint32_t i = 0; i < n_items; ++i) {

@@ -346,6 +346,8 @@ __global__ void __launch_bounds__(128, 7)
 constexpr uint64_t kQueueMinRays = 1u << 17;
 // Below this many rays, of which a fifth may enter the octree, too few are left per warp for flow_cast: random rays
 // on 256^3 take 125 us instead of 117 at 320,000, 164 instead of 166 at 640,000, 216 instead of 243 at 1,280,000.
+// Where all enter, flow_cast pays from about 200,000 rays (on 512^3 208 instead of 190 at 131,072, 262 instead of 310 at
+// 262,144): how many do is not known before the launch.
 constexpr uint64_t kFlowMinRays = 1u << 19;
 // From this many rays on plain_kernel's one block per SM less costs more than two launches: on 512^3 4.2 M camera rays take
 // 969 us in plain_kernel, 919 in launches of their own, 8.4 M 1,698 and 1,597, 8.4 M random ones 772 and 738; at 2.1 M both take
@@ -909,6 +911,9 @@ svo_status incremental_sync(svo_scene* sc, cudaStream_t st) {
 // rays, so that there are 4,096 warps or more (about what is resident).  A warp takes the sum of its rays' different
 // steps, so more warps of fewer rays end sooner while they all run at once: 4,000 camera rays on 128^3 take
 // 41 us instead of 97, 1,000 random ones 26 instead of 45, 60,000 on 512^3 106 instead of 147 in the work queue.
+// Not so from about 70,000 rays that all enter and go their own ways, which keep every resident warp busy: 100,000 on
+// 512^3 take 178 us with 16 rays a warp, 159 in the work queue, 149 with 32 a warp; of a camera's 124, 143 and 132,
+// of random ones of which a fifth enter 98, 104 and 103.
 constexpr uint64_t kGridWarps = 4096;
 uint32_t grid_lanes(uint64_t n) {
   uint32_t lanes = 5;
@@ -1121,7 +1126,7 @@ svo_status cast_host_pipelined(svo_scene* sc, const svo_rays* rays, uint64_t n, 
 }  // namespace
 
 // ------------------------------------------------------------------ LUT self-test kernel
-// Reports the tables exactly as a cast block holds them in shared memory.
+// Reports the tables exactly as a block of a staged cast holds them in shared memory (other casts read kLuts).
 __global__ void lut_kernel(uint64_t* rtn, uint32_t* step, uint64_t* mask) {
   __shared__ SharedLuts L;
   fill_shared_luts(L);

@@ -4,9 +4,10 @@
 // casts 32 of them to their ends, each kind of step in a loop of its own, runs 4 of 32 lanes (2^22 random rays on
 // 512^3: 905 M warp instructions, 1,015 us, bound by instruction issue).  Here a lane's ray is a small state
 // (Flow) that advances by a visit, a step or both per turn of one loop, and lanes whose rays have ended take new
-// ones: 10 of 32 lanes, 565 M warp instructions, 679 us.  The state is what bounds the form: at 72 registers
-// (7 blocks per SM) nothing of it may spill, so what is read rarely lives in shared memory, and what is a
-// function of the rest (the node's 1 / size, the direction's signs as masks) is formed again.
+// ones: 10 of 32 lanes, 526 M warp instructions, 635 us.  The state is what bounds the form: little of it may
+// spill, so what is read rarely lives in shared memory, and what is a function of the rest (the node's
+// 1 / size, the direction's signs as masks) is formed again.  It fits 72 registers (7 blocks per SM) in a
+// kernel of its own, 80 (6) beside queue_cast or with its scenes in a table.
 #pragma once
 
 #include "svo_unit.cuh"
@@ -505,7 +506,7 @@ svo_status launch_plain(const SceneView& v, const RaysView& rays, const HitsView
 
 // The first rays of the 32 pairs that rays_mixed looks at, one in each 32nd of the batch.  Where in it is scattered: at
 // equal distances the pairs of an image of 1920 x 1080 x 4 rays lay at 32 neighbouring columns, those at the row's end
-// with one ray on the next row, and its cast took 3.49 ms instead of 1.97.  Pairs are 8 apart, so that
+// with one ray on the next row, and its cast took 3.49 ms instead of 3.13.  Pairs are 8 apart, so that
 // few of them straddle a row's end from 64 columns on.
 constexpr uint32_t kPairApart = 8;
 SVO_UHD uint64_t pair_at(uint64_t n, uint32_t k) {
