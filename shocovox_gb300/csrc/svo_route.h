@@ -14,11 +14,10 @@ namespace svo {
 inline bool arrays_aligned(const svo_rays& rays, const svo_hits& hits) {
   const float* const in[6] = {rays.ox, rays.oy, rays.oz, rays.dx, rays.dy, rays.dz};
   void* const* out = reinterpret_cast<void* const*>(&hits);
-  for (const float* p : in)
-    if (reinterpret_cast<uintptr_t>(p) % sizeof(float)) return false;
-  for (int f = 0; f < kHitFields; ++f)
-    if (reinterpret_cast<uintptr_t>(out[f]) % kHitFieldBytes[f]) return false;
-  return true;
+  uintptr_t bits = 0;
+  for (const float* p : in) bits |= reinterpret_cast<uintptr_t>(p) & 3u;
+  for (int f = 0; f < kHitFields; ++f) bits |= reinterpret_cast<uintptr_t>(out[f]) & (kHitFieldBytes[f] - 1u);
+  return bits == 0;
 }
 
 // Whether hits written in place may change rays that are still to be read: a hit field over a ray array, other than element
@@ -26,9 +25,16 @@ inline bool arrays_aligned(const svo_rays& rays, const svo_hits& hits) {
 inline bool hits_over_rays(const svo_rays& rays, const svo_hits& hits, uint64_t n) {
   const float* const in[6] = {rays.ox, rays.oy, rays.oz, rays.dx, rays.dy, rays.dz};
   void* const* out = reinterpret_cast<void* const*>(&hits);
+  uintptr_t low = UINTPTR_MAX, high = 0;  // all rays lie between these
+  for (const float* p : in) {
+    const uintptr_t r = reinterpret_cast<uintptr_t>(p);
+    low = r < low ? r : low;
+    high = r > high ? r : high;
+  }
+  high += sizeof(float) * n;
   for (int f = 0; f < kHitFields; ++f) {
     const uintptr_t h = reinterpret_cast<uintptr_t>(out[f]);
-    if (!h) continue;
+    if (!h || h >= high || h + kHitFieldBytes[f] * n <= low) continue;
     for (const float* p : in) {
       const uintptr_t r = reinterpret_cast<uintptr_t>(p);
       if (h == r && kHitFieldBytes[f] == sizeof(float)) continue;
