@@ -14,18 +14,19 @@ NOISE = dict(seed=31, occupancy=0.08, spheres=3, octaves=2, base_freq=1.0 / 16, 
 
 
 class Items:
-    """Items of one call over (scene, origins, directions, row length); `check` compares them with the oracle."""
+    """Items of one call over (scene, origins, directions, row length[, the oracle's hits]); `check` compares them with the oracle."""
 
     def __init__(self, parts):
         self.items, self.keep = [], []
-        for (o, p), origins, dirs, row in parts:
+        for (o, p), origins, dirs, row, *ref in parts:
             n = len(origins)
+            ref = ref[0] if ref else o.cast(origins, dirs, threads=16) if n else None
             cols = {k: torch.from_numpy(np.ascontiguousarray(a[:, i])).cuda()
                     for a, names in ((origins, ("ox", "oy", "oz")), (dirs, ("dx", "dy", "dz"))) for i, k in enumerate(names)}
             out = {k: torch.zeros(n + 33, dtype=getattr(torch, np.dtype(svo.HIT_FIELDS[k]).name), device="cuda")
                    for k in UNCOUNTED}
             self.items.append((p, {k: v.data_ptr() for k, v in cols.items()}, n, {k: v.data_ptr() for k, v in out.items()}, row))
-            self.keep.append((cols, out, n, o.cast(origins, dirs, threads=16) if n else None))
+            self.keep.append((cols, out, n, ref))
 
     def clear(self):
         for _, out, _, _ in self.keep:
@@ -133,7 +134,7 @@ def odd_items(oracle_mod, seed):
         scene = both(oracle_mod, size, dim, svo.gen_scene(kind, size, dim, seed=seed + j, occupancy=0.1, spheres=3, octaves=2,
                                                           base_freq=1.0 / 16, height_lo=2.0, height_hi=size * 0.4))
         origins, dirs = special_rays(rng, size, n)
-        parts.append((scene, origins, dirs, row))
+        parts.append((scene, origins, dirs, row, scene[0].cast(origins, dirs, threads=16) if n else None))
     return parts
 
 
@@ -144,17 +145,17 @@ def cast_mode():
 
 
 def test_several_items(oracle_mod, cast_mode):
-    """Every launch configuration, both cast modes, two calls in a row; an item alone; no unordered item at all."""
+    """Launch configurations, both cast modes, one call after another on a workspace; an item alone; no unordered item at all."""
     parts = odd_items(oracle_mod, 700)
     ws = svo.BatchWorkspace()
     for mode in (0, 1):
         cast_mode(mode)
         items = Items(parts)
-        for cfg in ((0, 0, 0, 0, 1, 0, 0), (64, 32, 0, 0, 1, 2, 1), (128, 100, 0, 4, 1, 0, 8), (96, 256, 3, 0, 1, 4, 32),
-                    (32, 64, 1, 5, 1, 0, 24)):
-            for again in range(2):
-                items.cast(ws, svo.LaunchConfig(*cfg), "mode %d, %s, call %d" % (mode, cfg, again))
-        for only in ([4], [1], [2, 3], [5, 8], [2, 7, 9], [6, 0]):
+        configs = ((0, 0, 0, 0, 1, 0, 0), (64, 32, 0, 0, 1, 2, 1), (128, 100, 0, 4, 1, 0, 8), (96, 256, 3, 0, 1, 4, 32),
+                   (32, 64, 1, 5, 1, 0, 24))
+        for cfg in configs if mode == 0 else configs[:2]:  # rays that reach the work cap take a second a call
+            items.cast(ws, svo.LaunchConfig(*cfg), "mode %d, %s" % (mode, cfg))
+        for only in ([4], [1], [2, 3], [5, 8], [2, 7, 9], [6, 0]) if mode == 0 else ([1], [2, 3]):
             Items([parts[k] for k in only]).cast(ws, svo.LaunchConfig(0, 0, 0, 0, 1, 0, 0), "mode %d, items %s" % (mode, only))
 
 
